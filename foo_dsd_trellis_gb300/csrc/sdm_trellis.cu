@@ -27,6 +27,7 @@
 // act[] that lands on path_hash[0] while bank 1 is sorted (src/trellis.c:668-673).
 #include "sdm_internal.h"
 
+#include <algorithm>
 #include <climits>
 #include <cstdio>
 
@@ -70,6 +71,14 @@ __device__ __forceinline__ unsigned long long shfl64(unsigned long long v, int s
 // and handed to the surviving children as a Pack.  Each sample then keeps only
 // the s[0]-dependent operations on its critical path.  Every operation is the
 // reference's, in the reference's order, rounded separately (no contraction).
+//
+// A loop filter's resonators make every second g zero: the even ones for odd
+// orders, the odd ones for even orders (every filter of the table).  While
+// that holds and no value is infinite or NaN, g[i] s[i+1] is a zero and
+// subtracting it leaves its operand as it is (up to the sign of a zero, which
+// no cost depends on), so those products and differences are not issued: 35
+// of the 41 + 1 FP64 instructions of a step at order 7.  `zg` says that they
+// may be left out; a non-finite cost or state, or other g, takes them all.
 template <int N>
 struct Pack {
   double G0;      // g0 * s1
@@ -79,38 +88,93 @@ struct Pack {
 };
 
 template <int N>
-__host__ __device__ constexpr int shared_ops() { return N >= 3 ? 4 * N - 8 : 1; }
+__host__ __device__ constexpr bool g_zero(int i) { return (i & 1) == ((N & 1) ? 0 : 1); }
+
+// middle indices i = 2..N-2 with a nonzero g
+template <int N>
+__host__ __device__ constexpr int mid_g() {
+  int c = 0;
+  for (int i = 2; i <= N - 2; i++) c += g_zero<N>(i) ? 0 : 1;
+  return c;
+}
+
+template <int N>
+__host__ __device__ constexpr int shared_ops() {
+  return N >= 3 ? 1 + 2 * mid_g<N>() + (N - 3) + 1 + (N - 2) : 1;
+}
+
+// index of the k-th middle g that is not zero
+template <int N>
+__host__ __device__ constexpr int mid_g_at(int k) {
+  int c = 0;
+  for (int i = 2; i <= N - 2; i++)
+    if (!g_zero<N>(i)) {
+      if (c == k) return i;
+      c++;
+    }
+  return 2;
+}
 
 // Operation k of the shared part, inputs S[1..N-1] (a child's state), into
-// np (with scratch tg/tu).  Orders respect the dependencies when k runs
+// np (with scratch tg).  Orders respect the dependencies when k runs
 // 0, 1, 2, ...
 template <int N>
 __device__ __forceinline__ void shared_op(int k, const SdmParams& P, const double (&S)[N],
-                                          Pack<N>& np, double (&tg)[N], double (&tu)[N]) {
+                                          Pack<N>& np, double (&tg)[N], bool zg) {
   if (N < 3) {
     if (k == 0) np.G0 = __dmul_rn(P.g[0], S[1]);
     return;
   }
   constexpr int M = N - 3;   // middle indices i = 2..N-2
-  if (k == 0) { np.G0 = __dmul_rn(P.g[0], S[1]); return; }
-  if (k == 1) { np.G1 = __dmul_rn(P.g[1], S[2]); return; }
-  k -= 2;
-  if (k < M) { const int i = 2 + k; tg[i] = __dmul_rn(P.g[i], S[i + 1]); return; }
-  k -= M;
-  if (k < M) { const int i = 2 + k; tu[i] = __dadd_rn(S[i], S[i - 1]); return; }
+  constexpr int Z = mid_g<N>();
+  if (k == 0) {
+    if (g_zero<N>(0)) np.G1 = __dmul_rn(P.g[1], S[2]);
+    else np.G0 = __dmul_rn(P.g[0], S[1]);
+    return;
+  }
+  k -= 1;
+  if (k < Z) { const int i = mid_g_at<N>(k); tg[i] = __dmul_rn(P.g[i], S[i + 1]); return; }
+  k -= Z;
+  if (k < M) { const int i = 2 + k; np.D[i] = __dadd_rn(S[i], S[i - 1]); return; }
   k -= M;
   if (k == 0) { np.D[N - 1] = __dadd_rn(S[N - 1], S[N - 2]); return; }
   k -= 1;
-  if (k < M) { const int i = 2 + k; np.D[i] = __dsub_rn(tu[i], tg[i]); return; }
-  k -= M;
+  if (k < Z) { const int i = mid_g_at<N>(k); np.D[i] = __dsub_rn(np.D[i], tg[i]); return; }
+  k -= Z;
+  if (k == 0 && !zg) {
+    // the products with the g that are zero in the table's filters
+    if (g_zero<N>(0)) np.G0 = __dmul_rn(P.g[0], S[1]);
+    else np.G1 = __dmul_rn(P.g[1], S[2]);
+#pragma unroll
+    for (int i = 2; i <= N - 2; i++)
+      if (g_zero<N>(i)) np.D[i] = __dsub_rn(np.D[i], __dmul_rn(P.g[i], S[i + 1]));
+  }
   if (k < N - 2) { const int i = 2 + k; np.A[i] = __dmul_rn(P.a[i], np.D[i]); return; }
 }
 
 template <int N>
-__device__ __forceinline__ void shared_all(const SdmParams& P, const double (&S)[N], Pack<N>& np) {
-  double tg[N], tu[N];
+__device__ __forceinline__ void shared_all(const SdmParams& P, const double (&S)[N], Pack<N>& np,
+                                           bool zg) {
+  double tg[N];
 #pragma unroll
-  for (int k = 0; k < shared_ops<N>(); k++) shared_op<N>(k, P, S, np, tg, tu);
+  for (int k = 0; k < shared_ops<N>(); k++) shared_op<N>(k, P, S, np, tg, zg);
+}
+
+// Whether this filter's g has the zero pattern and no a is zero (a state that
+// is not finite then always shows in a cost that is not finite).
+__device__ __forceinline__ bool zero_pattern(const SdmParams& P, int N) {
+  bool ok = true;
+  for (int i = 0; i < N; i++) {
+    const long long a = __double_as_longlong(P.a[i]) & 0x7fffffffffffffffll;
+    const long long g = __double_as_longlong(P.g[i]) & 0x7fffffffffffffffll;
+    if (a == 0 || a >= 0x7ff0000000000000ll || g >= 0x7ff0000000000000ll) ok = false;
+    if (i <= N - 2 && (i & 1) == ((N & 1) ? 0 : 1) && g != 0) ok = false;
+  }
+  return ok;
+}
+
+__device__ __forceinline__ bool not_finite(double v) {
+  return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u;
 }
 
 // Shared memory of one job run by LPJ lanes: the slot memory of both banks
@@ -128,6 +192,11 @@ struct WarpSmem {
   uint8_t hashmark2[S];        // children the fast path deems hashed
   int8_t pos[S];               // sorted position of each child (serial path)
   int8_t idx_at[S];            // child at each sorted position (serial path)
+  // lanes by path, for the search of equal paths: 64 entries a lane, so that
+  // two different paths seldom share one (32 lanes, 2,048 entries: 0.24 pairs
+  // a sample)
+  static constexpr int kTab = 64 * LPJ;
+  uint8_t tab[kTab];
 };
 
 // Lanes per job: the smallest power of two >= K (at least 2) is the tightest
@@ -160,21 +229,20 @@ static int resident_warps() {
   return cached[dev];
 }
 
-// Lanes for a launch of njobs jobs with no block cap: the widest width whose
-// jobs all fit in one wave of resident warps.  The trellis step of a small-K
-// job is bound by its serial selection chain rather than by FP64 issue, so
-// fewer jobs per warp run faster as long as no job waits for a second wave
-// (10 s stereo same-rate DSD128, 1722 jobs: K = 16 at 32 lanes 289 vs 256 at
-// 16 lanes DSD Msamples/s; K = 2 at 2 lanes 174, at 16 lanes 309).
-static int launch_lanes(const SdmParams& P, int njobs, int max_blocks) {
-  if (P.lanes > 0 || max_blocks > 0 || P.lat > 32 * kRegRingWords) return lanes_per_job(P);
-  const int lo = min_lanes(P.cands);
-  int lanes = 32;
-  // warp slots of a width: 16 one-warp CTAs per SM at 32 lanes (128 registers),
-  // 10 below (their launch bound leaves up to 204 registers)
-  while (lanes > lo &&
-         (long long)njobs * lanes > (long long)resident_warps() / 16 * (lanes == 32 ? 16 : 10) * 32)
-    lanes >>= 1;
+// Lanes and jobs per warp of a launch of njobs jobs with no block cap: the
+// tightest width, and the fewest jobs a warp that still let every job start at
+// once (warp slots: 16 one-warp CTAs per SM at 32 lanes, 10 below, whose launch
+// bound leaves up to 204 registers).  The selection's sort is as deep as the
+// width asks (21 exchanges at 32 lanes, 15 at 16, 10 at 8), and an FP64
+// instruction costs the same with 8 lanes active as with 32, so idle lanes
+// beside a job cost nothing while a second job on them costs its FP64 time.
+static int launch_lanes(const SdmParams& P, int njobs, int max_blocks, int* groups) {
+  int lanes = lanes_per_job(P);
+  *groups = 32 / lanes;
+  if (P.lanes > 0 || max_blocks > 0 || P.lat > 32 * kRegRingWords) return lanes;
+  lanes = min_lanes(P.cands);
+  const long long slots = (long long)(resident_warps() / 16) * (lanes == 32 ? 16 : 10);
+  *groups = (int)std::min<long long>(32 / lanes, std::max<long long>(1, (njobs + slots - 1) / slots));
   return lanes;
 }
 
@@ -188,19 +256,65 @@ __device__ __forceinline__ bool key_less(long long ka, int ia, long long kb, int
   return ka < kb || (ka == kb && ia < ib);
 }
 
-// Bitonic sort of the 2 * LPJ (key, index) pairs of one job, two per lane
-// (sorted positions 2*lane and 2*lane + 1), ascending.  With LPJ = 16 each
-// half-warp sorts its own job (exchange distances stay inside the half).
+// A child's cost and index as one 32-bit word: 26 bits of the cost (its key
+// from 2^-24 to 2^8 in 2^21 steps an octave, clamped outside) over 6 bits of
+// index.  Words order like (key, index) wherever their cost parts differ.
+constexpr unsigned kWordBase = (1023u - 24u) << 21;
+constexpr unsigned kWordTop = 0x3fffffeu;    // largest cost part of a child
+constexpr unsigned kWordNone = 0x3ffffffu;   // no child
+
+__device__ __forceinline__ unsigned key_word(long long key, int idx) {
+  const unsigned hi = (unsigned)((unsigned long long)key >> 32);
+  const unsigned u = __funnelshift_l((unsigned)key, hi, 1);   // key >> 31 for keys >= 0
+  const unsigned w = min(max(u, kWordBase) - kWordBase, kWordTop);
+  return (w << 6) | (unsigned)idx;
+}
+
+// Bitonic sort of the 2 * LPJ words of one job, two per lane (sorted positions
+// 2*lane and 2*lane + 1), ascending: each merge starts with the mirrored
+// exchange, so every exchange keeps the smaller word at the lower position.
 template <int LPJ, typename Hook>
-__device__ __forceinline__ void bitonic_sort(long long& kA, int& iA, long long& kB, int& iB,
-                                             int lane, unsigned hm, Hook&& hook) {
+__device__ __forceinline__ void word_sort(unsigned& c0, unsigned& c1, int lane, unsigned hm,
+                                          Hook&& hook) {
   int stage = 0;
 #pragma unroll
   for (int k = 2; k <= 2 * LPJ; k <<= 1) {
-    const bool asc = ((2 * lane) & k) == 0;
+    hook(stage++);
+    if (k > 2) {
+      const bool low = (lane & (k >> 2)) == 0;
+      const unsigned p1 = __shfl_xor_sync(hm, c1, (k >> 1) - 1, LPJ);
+      const unsigned p0 = __shfl_xor_sync(hm, c0, (k >> 1) - 1, LPJ);
+      c0 = low ? min(c0, p1) : max(c0, p1);
+      c1 = low ? min(c1, p0) : max(c1, p0);
 #pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int j = k >> 2; j > 1; j >>= 1) {
+        hook(stage++);
+        const bool lo = (lane & (j >> 1)) == 0;
+        const unsigned q0 = __shfl_xor_sync(hm, c0, j >> 1, LPJ);
+        const unsigned q1 = __shfl_xor_sync(hm, c1, j >> 1, LPJ);
+        c0 = lo ? min(c0, q0) : max(c0, q0);
+        c1 = lo ? min(c1, q1) : max(c1, q1);
+      }
       hook(stage++);
+    }
+    const unsigned mn = min(c0, c1), mx = max(c0, c1);
+    c0 = mn;
+    c1 = mx;
+  }
+}
+
+// The same order by the whole (key, index) pairs, for the samples whose words
+// do not tell (two children within 2^-21 of each other's cost, a cost out of
+// the words' range, or one that is not finite).  Not unrolled: it is rare, and
+// its code stays out of the step loop's registers.
+template <int LPJ>
+__device__ __forceinline__ void full_sort(long long& kA, int& iA, long long& kB, int& iB, int lane,
+                                          unsigned hm) {
+#pragma unroll 1
+  for (int k = 2; k <= 2 * LPJ; k <<= 1) {
+    const bool asc = ((2 * lane) & k) == 0;
+#pragma unroll 1
+    for (int j = k >> 1; j > 0; j >>= 1) {
       if (j == 1) {
         const bool sw = asc ? key_less(kB, iB, kA, iA) : key_less(kA, iA, kB, iB);
         if (sw) {
@@ -296,10 +410,35 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     }
     __syncwarp(hm);
   }
+  // the products with the filter's zero g are left out while every value is
+  // finite (see Pack)
+  bool zg = zero_pattern(P, N);
+  {
+    bool nf = false;
+#pragma unroll
+    for (int k = 0; k < N; k++) nf |= not_finite(s[k]);
+    if (__any_sync(hm, nf)) zg = false;
+  }
   // the candidate as (s0, s1, shared part of its next advance)
   double cs0 = s[0], cs1 = s[1];
   Pack<N> pk;
-  shared_all<N>(P, s, pk);
+  pk.G0 = pk.G1 = 0.0;
+  shared_all<N>(P, s, pk, zg);
+
+  // the traceback ring's word being written, and for the other words the lane
+  // whose ring they were when that word was entered: they are moved between
+  // lanes once per word, not once per sample
+  uint32_t cur = 0;
+#pragma unroll
+  for (int w = 0; w < RW; w++) {
+    const uint32_t r = reg_word<RW>(ring[w]);
+    if (w == (pos >> 5)) cur = r;
+  }
+  int perm = lane;
+  // equal paths are searched by a table of paths: the path itself where the
+  // masked paths number no more than its entries
+  constexpr int kTabBits = LPJ == 32 ? 11 : LPJ == 16 ? 10 : LPJ == 8 ? 9 : LPJ == 4 ? 8 : 7;
+  const bool tab_direct = P.depth - 1 <= kTabBits;
 
   const long long n_in = job.n_in;
   const double* __restrict__ in = job.in;
@@ -323,152 +462,226 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     int next_pos = pos + 1;
     if (next_pos == P.lat) next_pos = 0;
     const bool live = lane < n;
+    const unsigned livemask = n >= 32 ? 0xffffffffu : ((1u << n) - 1u);
+    // only at K = 32 while bank 1 is sorted can a slot's path, cost and chain
+    // link be read in a later sample (see the selection)
+    const bool links_matter = (K == kMaxCands && nb == 1);
 
     // ---- 1. expansion: the s0-dependent part of the advance ----
+    const unsigned long long q = (path << 1) & mask;
     double S[N];          // the children's shared state s[1..N-1] (clamped)
+    S[0] = 0.0;
+    const double d0 = __dadd_rn(g_zero<N>(0) && zg ? cs0 : __dsub_rn(cs0, pk.G0), x);
+    double d1 = __dadd_rn(cs1, cs0);
+    if (N >= 3 && !(g_zero<N>(1) && zg)) d1 = __dsub_rn(d1, pk.G1);
+    double v = __dadd_rn(x, __dmul_rn(P.a[0], d0));
+    v = __dadd_rn(v, __dmul_rn(P.a[1], d1));
+
+    // equal paths: children of two candidates share a path iff their q are
+    // equal.  Every live lane leaves its number at its path's table entry; a
+    // lane that reads another's number there compares the paths, and a second
+    // round tells the other lane.  More than one such lane at one entry takes
+    // the warp's match instruction, which costs 270 to 510 cycles (measured)
+    // and used to run on every sample.
+    int partner = -1;       // the live lane with this lane's q
+    bool multi = false;     // three or more live lanes share a q
+    unsigned ti;
+    if (tab_direct) {
+      ti = (unsigned)(q >> 1) & (WarpSmem<LPJ>::kTab - 1);
+    } else {
+      const unsigned m = ((unsigned)q + (unsigned)(q >> 32) * 0x85ebca77u) * 0x9e3779b1u;
+      ti = m >> (32 - kTabBits);
+    }
+    if (live) sm.tab[ti] = (uint8_t)lane;
+    const unsigned nx1 = BALLOT(live && nxt);   // traceback bits of the candidates
+    __syncwarp(hm);
+    const int holder = live ? (int)sm.tab[ti] : lane;
+    const bool pany = __any_sync(hm, holder != lane);
+
 #pragma unroll
-    for (int k = 0; k < N; k++) S[k] = 0.0;
-    double s00 = 0.0, s01 = 0.0;
-    long long key0 = LLONG_MAX, key1 = LLONG_MAX;
-    unsigned long long q = 0;
-    int new_next = 0;
-    const int old_next = nxt;
-    if (live) {
-      const double d0 = __dadd_rn(__dsub_rn(cs0, pk.G0), x);
-      const double d1 = (N >= 3) ? __dsub_rn(__dadd_rn(cs1, cs0), pk.G1) : __dadd_rn(cs1, cs0);
-      double v = __dadd_rn(x, __dmul_rn(P.a[0], d0));
-      v = __dadd_rn(v, __dmul_rn(P.a[1], d1));
+    for (int i = 2; i < N; i++) v = __dadd_rn(v, pk.A[i]);
+    S[1] = d1;
 #pragma unroll
-      for (int i = 2; i < N; i++) v = __dadd_rn(v, pk.A[i]);
-      s00 = __dadd_rn(d0, 1.0);
-      s01 = __dsub_rn(d0, 1.0);
-      S[1] = d1;
+    for (int i = 2; i < N; i++) S[i] = pk.D[i];
+    if (lim_on) {
 #pragma unroll
-      for (int i = 2; i < N; i++) S[i] = pk.D[i];
-      if (lim_on) {
-#pragma unroll
-        for (int k = 1; k < N; k++) S[k] = clamp_state(S[k], P.state_limit);
-        s00 = clamp_state(s00, P.state_limit);
-        s01 = clamp_state(s01, P.state_limit);
+      for (int k = 1; k < N; k++) S[k] = clamp_state(S[k], P.state_limit);
+    }
+    if (pany) {
+      const unsigned long long qh = shfl64<LPJ>(q, holder, hm);
+      const bool lose = holder != lane;
+      __syncwarp(hm);
+      if (lose) sm.tab[ti] = (uint8_t)lane;
+      __syncwarp(hm);
+      const int second = live ? (int)sm.tab[ti] : lane;
+      const unsigned long long q2 = shfl64<LPJ>(q, second, hm);
+      if (__any_sync(hm, lose && second != lane)) {
+        const unsigned mm = MATCH(live ? q : ~(unsigned long long)lane) & livemask;
+        const unsigned oth = mm & ~(1u << lane);
+        if (live && __popc(mm) == 2) partner = __ffs(oth) - 1;
+        multi = __any_sync(hm, live && __popc(mm) > 2);
+      } else if (lose) {
+        if (qh == q) partner = holder;
+      } else if (live && second != lane && q2 == q) {
+        partner = second;
       }
-      const double e0 = __dadd_rn(v, P.a[0]);
-      const double e1 = __dsub_rn(v, P.a[0]);
-      key0 = key_of(__dadd_rn(cost, __dmul_rn(e0, e0)));
-      key1 = key_of(__dadd_rn(cost, __dmul_rn(e1, e1)));
-      q = (path << 1) & mask;
-      uint32_t wv = 0;
+    }
+    // the parent's traceback bit at next_pos
+    uint32_t wv = cur;
+    const bool cross = (next_pos >> 5) != (pos >> 5);
+    if (cross) {
 #pragma unroll
       for (int w = 0; w < RW; w++) {
         const uint32_t r = reg_word<RW>(ring[w]);
         if (w == (next_pos >> 5)) wv = r;
       }
-      new_next = (int)((wv >> (next_pos & 31)) & 1u);
-      sm.path[nb][2 * lane] = q;
-      sm.path[nb][2 * lane + 1] = q | 1ull;
+      wv = __shfl_sync(hm, wv, perm, LPJ);
+    }
+    const int new_next = (int)((wv >> (next_pos & 31)) & 1u);
+
+    const double e0 = __dadd_rn(v, P.a[0]);
+    const double e1 = __dsub_rn(v, P.a[0]);
+    const long long key0 = key_of(__dadd_rn(cost, __dmul_rn(e0, e0)));
+    const long long key1 = key_of(__dadd_rn(cost, __dmul_rn(e1, e1)));
+    if (live) {
       sm.key[nb][2 * lane] = key0;
       sm.key[nb][2 * lane + 1] = key1;
-      sm.heads[q & (kBuckets - 1)] = -1;
-      sm.heads[(q | 1ull) & (kBuckets - 1)] = -1;
+      if (links_matter) {
+        sm.path[nb][2 * lane] = q;
+        sm.path[nb][2 * lane + 1] = q | 1ull;
+      }
     }
-    __syncwarp(hm);
+    const bool odd_key = live && ((unsigned)(key0 >> 32) >= 0x7ff00000u ||
+                                  (unsigned)(key1 >> 32) >= 0x7ff00000u);
+    const bool bad = __any_sync(hm, odd_key);
+    if (bad) zg = false;   // the shared part below takes every product
 
-    // the children's shared part, one operation per stage of the sort below
+    // the children's shared part, spread over the sort's stages below
     Pack<N> npk;
-    double tg[N], tu[N];
+    double tg[N];
     // ---- 2. selection ----
     // All 2n children sorted by (cost bits as int64, slot index): position 0
     // is the reference's minimum (first index among equal costs), the first
     // sorted child carrying the majority bit is its best_maj, and the
     // eligible children keep their (cost, index) order (src/trellis.c:628-652).
-    long long sk0 = live ? key0 : LLONG_MAX, sk1 = live ? key1 : LLONG_MAX;
-    int si0 = 2 * lane, si1 = 2 * lane + 1;
+    // The sort runs on 32-bit words (key_word): one shuffle and one min / max
+    // an exchange where the whole (key, index) pairs took three shuffles and a
+    // 64-bit comparison (1,000 of a step's 7,400 cycles).
+    unsigned c0 = live ? key_word(key0, 2 * lane) : (kWordNone << 6) | (unsigned)(2 * lane);
+    unsigned c1 = live ? key_word(key1, 2 * lane + 1) : (kWordNone << 6) | (unsigned)(2 * lane + 1);
     // The shared-part operations ride on the sort stages, except the last
     // kDeferOps, which are issued at the start of the selection so that its
     // integer work runs while they occupy the FP64 unit.
     constexpr int kOps = shared_ops<N>();
     constexpr int kStages = sort_stages<LPJ>();
-    constexpr int kDeferOps = 8;
+    constexpr int kDeferOps = 6;
     constexpr int kSortOps = (kOps < kStages ? kOps : kStages) > kDeferOps
                                  ? (kOps < kStages ? kOps : kStages) - kDeferOps : 0;
-    bitonic_sort<LPJ>(sk0, si0, sk1, si1, lane, hm, [&](int st) {
-      if (st < kSortOps) shared_op<N>(st, P, S, npk, tg, tu);
+    word_sort<LPJ>(c0, c1, lane, hm, [&](int st) {
+      if (st < kSortOps) shared_op<N>(st, P, S, npk, tg, zg);
     });
-    const int sn0 = __shfl_sync(hm, old_next, si0 >> 1, LPJ);   // traceback bit of each sorted child
-    const int sn1 = __shfl_sync(hm, old_next, si1 >> 1, LPJ);
+    int si0 = (int)(c0 & 63u), si1 = (int)(c1 & 63u);
+    {
+      const unsigned after = __shfl_down_sync(hm, c0, 1, LPJ);
+      const bool same = (c0 >> 6) == (c1 >> 6) && (c1 >> 6) != kWordNone;
+      const bool same2 = lane < LPJ - 1 && (c1 >> 6) == (after >> 6) && (c1 >> 6) != kWordNone;
+      if (__any_sync(hm, same || same2) || bad) {
+        long long sk0 = live ? key0 : LLONG_MAX, sk1 = live ? key1 : LLONG_MAX;
+        si0 = 2 * lane;
+        si1 = 2 * lane + 1;
+        full_sort<LPJ>(sk0, si0, sk1, si1, lane, hm);
+      }
+    }
     const bool sl0 = (si0 >> 1) < n, sl1 = (si1 >> 1) < n;
-    const unsigned nx1 = BALLOT(live && old_next);
+    const int sn0 = (int)((nx1 >> (si0 >> 1)) & 1u);   // traceback bit of each sorted child
+    const int sn1 = (int)((nx1 >> (si1 >> 1)) & 1u);
     const int votes1 = 2 * __popc(nx1);
     const int majority = (votes1 > 2 * n - votes1) ? 1 : 0;
-    const long long mk = __shfl_sync(hm, sk0, 0, LPJ);
-    int want = __shfl_sync(hm, sn0, 0, LPJ);
+    const int first = __shfl_sync(hm, si0, 0, LPJ);
+    int want = (int)((nx1 >> (first >> 1)) & 1u);
     if (want != majority) {
+      __syncwarp(hm);
       const unsigned mA = BALLOT(sl0 && sn0 == majority);
       const unsigned mB = BALLOT(sl1 && sn1 == majority);
-      int pos = 1 << 20;
-      if (mA) pos = 2 * (__ffs(mA) - 1);
-      if (mB) pos = min(pos, 2 * (__ffs(mB) - 1) + 1);
-      if (pos < (1 << 20)) {
-        const long long bA = __shfl_sync(hm, sk0, pos >> 1, LPJ);
-        const long long bB = __shfl_sync(hm, sk1, pos >> 1, LPJ);
-        const double cbm = __longlong_as_double((pos & 1) ? bB : bA);
-        if (cbm < __dmul_rn(__longlong_as_double(mk), 1.1)) want = majority;
+      int at = 1 << 20;
+      if (mA) at = 2 * (__ffs(mA) - 1);
+      if (mB) at = min(at, 2 * (__ffs(mB) - 1) + 1);
+      if (at < (1 << 20)) {
+        const int bA = __shfl_sync(hm, si0, at >> 1, LPJ);
+        const int bB = __shfl_sync(hm, si1, at >> 1, LPJ);
+        const double cbm = __longlong_as_double(sm.key[nb][(at & 1) ? bB : bA]);
+        if (cbm < __dmul_rn(__longlong_as_double(sm.key[nb][first]), 1.1)) want = majority;
       }
     }
 #pragma unroll
-    for (int k = kSortOps; k < kOps; k++) shared_op<N>(k, P, S, npk, tg, tu);
-    unsigned elig = BALLOT(live && old_next == want);
+    for (int k = kSortOps; k < kOps; k++) shared_op<N>(k, P, S, npk, tg, zg);
+    const unsigned elig = want ? nx1 : (livemask & ~nx1);
     c_drop += 2ull * (unsigned)(n - __popc(elig));
     c_tot += 2ull * (unsigned)n;
 
     // ---- 2b. fast selection ----
-    // With no two eligible children on the same path, the reference's ordered
-    // insertion with path-hash dedup keeps exactly the first K eligible
-    // children of the (cost, index) order: every insert is new to the hash,
-    // evictions drop the largest, ties keep insertion (index) order, skips are
-    // children that would not be among the K smallest.  A child is hashed iff
-    // fewer than K eligible children with a lower index precede it in that
-    // order; only at K = 32 while bank 1 is sorted can the stored chain links
-    // be read in a later sample (through the act[32] store onto path_hash[0]),
-    // so only then are they written, as "previous hashed child of the same
-    // bucket".  Duplicate paths, or a bucket-0 child once the list can be full
-    // at K = 32 in bank 1, take the serial path.
-    const bool me = live && old_next == want;
-    const bool e0 = sl0 && sn0 == want, e1 = sl1 && sn1 == want;
-    const unsigned EA = BALLOT(e0), EB = BALLOT(e1);
+    // Without equal paths, the reference's ordered insertion with path-hash
+    // dedup keeps exactly the first K eligible children of the (cost, index)
+    // order: every insert is new to the hash, evictions drop the largest, ties
+    // keep insertion (index) order, skips are children that would not be among
+    // the K smallest.  Where two candidates share a q, of each pair of children
+    // with one path only the first in that order stays: the later one either
+    // finds it hashed, or replaces it, or finds it gone because the list's
+    // worst was better already.  (Three or more on one path keep their reference
+    // order in the serial path: a child replaced there stays in the hash.)
+    // A child is hashed iff fewer than K eligible children with a lower index
+    // precede it in that order; only at K = 32 while bank 1 is sorted can the
+    // stored chain links be read in a later sample (through the act[32] store
+    // onto path_hash[0]), so only then are they written, as "previous hashed
+    // child of the same bucket".  There, equal paths, or a bucket-0 child once
+    // the list can be full, take the serial path.
+    const bool me = live && ((elig >> lane) & 1u);
+    bool fast_ok = (P.mode != kModeExact) && !multi;
+    unsigned rem0 = 0u, rem1 = 0u;   // lanes whose child 0 / 1 loses to its equal
+    if (pany) {
+      const bool dup = me && partner >= 0 && ((elig >> (partner & 31)) & 1u);
+      if (links_matter) {
+        if (__any_sync(hm, dup)) fast_ok = false;
+      } else {
+        const int ps = partner >= 0 ? partner : lane;
+        const long long o0 = (long long)shfl64<LPJ>((unsigned long long)key0, ps, hm);
+        const long long o1 = (long long)shfl64<LPJ>((unsigned long long)key1, ps, hm);
+        rem0 = BALLOT(dup && key_less(o0, ps, key0, lane));
+        rem1 = BALLOT(dup && key_less(o1, ps, key1, lane));
+      }
+    }
+    const bool f0 = sl0 && ((elig >> (si0 >> 1)) & 1u) &&
+                    !((((si0 & 1) ? rem1 : rem0) >> (si0 >> 1)) & 1u);
+    const bool f1 = sl1 && ((elig >> (si1 >> 1)) & 1u) &&
+                    !((((si1 & 1) ? rem1 : rem0) >> (si1 >> 1)) & 1u);
+    const unsigned EA = BALLOT(f0), EB = BALLOT(f1);
     const int m2 = __popc(EA) + __popc(EB);
-    const bool links_matter = (K == kMaxCands && nb == 1);
-    bool fast_ok = (P.mode != kModeExact);
     int f_cnt = 0, f_Ls = -1, f_link0 = -1, f_link1 = -1;
     long long f_Lk = LLONG_MAX;
     bool f_h0 = false, f_h1 = false;
-    if (fast_ok) {
-      const unsigned mm = MATCH(q);
-      if (__any_sync(hm, me && __popc(mm & elig) > 1)) fast_ok = false;
-      if (links_matter && m2 > K && __any_sync(hm, me && (q & (kBuckets - 1)) == 0))
-        fast_ok = false;
-    }
+    if (links_matter && m2 > K && __any_sync(hm, me && (q & (kBuckets - 1)) == 0)) fast_ok = false;
     if (fast_ok) {
       const unsigned below = (1u << lane) - 1u;
       const int r0 = __popc(EA & below) + __popc(EB & below);
-      const int r1 = r0 + (e0 ? 1 : 0);
-      if (e0 && r0 < K) sm.act[r0] = (int8_t)si0;
-      if (e1 && r1 < K) sm.act[r1] = (int8_t)si1;
+      const int r1 = r0 + (f0 ? 1 : 0);
+      if (f0 && r0 < K) sm.act[r0] = (int8_t)si0;
+      if (f1 && r1 < K) sm.act[r1] = (int8_t)si1;
       if (links_matter) {
         // eligible children sorted before, with a lower index: OR-scan of
         // one-hot index masks over the sorted positions
-        const unsigned long long mine = (e0 ? (1ull << si0) : 0ull) | (e1 ? (1ull << si1) : 0ull);
+        const unsigned long long mine = (f0 ? (1ull << si0) : 0ull) | (f1 ? (1ull << si1) : 0ull);
         unsigned long long inc = mine;
 #pragma unroll
         for (int o = 1; o < LPJ; o <<= 1) {
-          const unsigned long long v = (unsigned long long)__shfl_up_sync(hm, (long long)inc, o, LPJ);
-          if (lane >= o) inc |= v;
+          const unsigned long long u = (unsigned long long)__shfl_up_sync(hm, (long long)inc, o, LPJ);
+          if (lane >= o) inc |= u;
         }
         const unsigned long long before0 = inc & ~mine;
-        const unsigned long long before1 = before0 | (e0 ? (1ull << si0) : 0ull);
+        const unsigned long long before1 = before0 | (f0 ? (1ull << si0) : 0ull);
         const int p0 = __popcll(before0 & ((1ull << si0) - 1ull));
         const int p1 = __popcll(before1 & ((1ull << si1) - 1ull));
-        sm.hashmark2[si0] = (uint8_t)(e0 && p0 < K);
-        sm.hashmark2[si1] = (uint8_t)(e1 && p1 < K);
+        sm.hashmark2[si0] = (uint8_t)(f0 && p0 < K);
+        sm.hashmark2[si1] = (uint8_t)(f1 && p1 < K);
       }
       __syncwarp(hm);
       f_cnt = m2 < K ? m2 : K;
@@ -480,8 +693,18 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
         f_h0 = live && sm.hashmark2[2 * lane] != 0;
         f_h1 = live && sm.hashmark2[2 * lane + 1] != 0;
         const unsigned H0 = BALLOT(f_h0), H1 = BALLOT(f_h1);
-        const unsigned s0 = MATCH((unsigned)(q & (kBuckets - 1))) & H0 & below;
-        const unsigned s1 = MATCH((unsigned)((q | 1ull) & (kBuckets - 1))) & H1 & below;
+        // lanes whose children fall in this lane's buckets (bits 1..6 of q; the
+        // children of bit 0 and 1 have a bucket each): one ballot per bit
+        unsigned bm = 0xffffffffu;
+#pragma unroll
+        for (int k = 1; k < 7; k++) {
+          const bool on = ((unsigned)q >> k) & 1u;
+          const unsigned bb = __ballot_sync(hm, on);
+          bm &= on ? bb : ~bb;
+        }
+        bm >>= sh;
+        const unsigned s0 = bm & H0 & below;
+        const unsigned s1 = bm & H1 & below;
         f_link0 = s0 ? 2 * (31 - __clz(s0)) : -1;
         f_link1 = s1 ? 2 * (31 - __clz(s1)) + 1 : -1;
       }
@@ -503,6 +726,13 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       sm.pos[si1] = (int8_t)(2 * lane + 1);
       sm.idx_at[2 * lane] = (int8_t)si0;
       sm.idx_at[2 * lane + 1] = (int8_t)si1;
+      if (live) {
+        // every lookup below is in a bucket of this sample's children
+        sm.path[nb][2 * lane] = q;
+        sm.path[nb][2 * lane + 1] = q | 1ull;
+        sm.heads[q & (kBuckets - 1)] = -1;
+        sm.heads[(q | 1ull) & (kBuckets - 1)] = -1;
+      }
       if (P.mode == kModeVerify && live) { sm.hashmark[2 * lane] = 0; sm.hashmark[2 * lane + 1] = 0; }
       __syncwarp(hm);
       const int nch = 2 * n;
@@ -575,14 +805,14 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
 
     if (fast_ok) {
       if (P.mode == kModeVerify) {
-        bool bad = (cnt != f_cnt) || (lane < cnt && (Ls != f_Ls || Lk != f_Lk));
+        bool vbad = (cnt != f_cnt) || (lane < cnt && (Ls != f_Ls || Lk != f_Lk));
         if (links_matter) {
-          if (live && (sm.hashmark[2 * lane] != 0) != f_h0) bad = true;
-          if (live && (sm.hashmark[2 * lane + 1] != 0) != f_h1) bad = true;
-          if (f_h0 && sm.link[nb][2 * lane] != f_link0) bad = true;
-          if (f_h1 && sm.link[nb][2 * lane + 1] != f_link1) bad = true;
+          if (live && (sm.hashmark[2 * lane] != 0) != f_h0) vbad = true;
+          if (live && (sm.hashmark[2 * lane + 1] != 0) != f_h1) vbad = true;
+          if (f_h0 && sm.link[nb][2 * lane] != f_link0) vbad = true;
+          if (f_h1 && sm.link[nb][2 * lane + 1] != f_link1) vbad = true;
         }
-        if (__any_sync(hm, bad)) err = max(err, (int)kStatusVerifyMismatch);
+        if (__any_sync(hm, vbad)) err = max(err, (int)kStatusVerifyMismatch);
       } else {
         cnt = f_cnt;
         Ls = f_Ls;
@@ -591,7 +821,6 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
           if (f_h0) sm.link[nb][2 * lane] = (int8_t)f_link0;
           if (f_h1) sm.link[nb][2 * lane + 1] = (int8_t)f_link1;
         }
-        __syncwarp(hm);
       }
     }
 
@@ -602,55 +831,58 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     const bool surv = lane < n_new;
     const int pp = surv ? (Ls >> 1) : lane;
     const int hh = surv ? (Ls & 1) : 0;
-    const double f00 = __shfl_sync(hm, s00, pp, LPJ);
-    const double f01 = __shfl_sync(hm, s01, pp, LPJ);
+    const double fd0 = __shfl_sync(hm, d0, pp, LPJ);
     const double fS1 = __shfl_sync(hm, S[1], pp, LPJ);
-    Pack<N> fp;
-    fp.G0 = __shfl_sync(hm, npk.G0, pp, LPJ);
-    if (N >= 3) fp.G1 = __shfl_sync(hm, npk.G1, pp, LPJ);
+    if (N < 3 || !(g_zero<N>(0) && zg)) pk.G0 = __shfl_sync(hm, npk.G0, pp, LPJ);
+    if (N >= 3 && !(g_zero<N>(1) && zg)) pk.G1 = __shfl_sync(hm, npk.G1, pp, LPJ);
 #pragma unroll
     for (int i = 2; i < N; i++) {
-      fp.D[i] = __shfl_sync(hm, npk.D[i], pp, LPJ);
-      fp.A[i] = __shfl_sync(hm, npk.A[i], pp, LPJ);
+      pk.D[i] = __shfl_sync(hm, npk.D[i], pp, LPJ);
+      pk.A[i] = __shfl_sync(hm, npk.A[i], pp, LPJ);
     }
-    const bool last = (t == n_in - 1);
-    double fs[N];
-    if (last) {
+    // the child's own s0 (both siblings share d0)
+    cs0 = __dadd_rn(fd0, hh ? -1.0 : 1.0);
+    if (lim_on) cs0 = clamp_state(cs0, P.state_limit);
+    cs1 = fS1;
+    if (t == n_in - 1) {
       // the full child state is only needed when the context is stored
-#pragma unroll
-      for (int i = 2; i < N; i++) fs[i] = __shfl_sync(hm, S[i], pp, LPJ);
-    }
-    const unsigned long long npath = shfl64<LPJ>(q, pp, hm) | (unsigned long long)hh;
-    const int nnext = __shfl_sync(hm, new_next, pp, LPJ);
-    uint32_t nring[RW];
-#pragma unroll
-    for (int w = 0; w < RW; w++)
-      nring[w] = (w < W) ? __shfl_sync(hm, ring[w], pp, LPJ) : 0u;
-    if (surv) {
-      cs0 = hh ? f01 : f00;
-      cs1 = fS1;
-      pk.G0 = fp.G0;
-      if (N >= 3) pk.G1 = fp.G1;
-#pragma unroll
-      for (int i = 2; i < N; i++) { pk.D[i] = fp.D[i]; pk.A[i] = fp.A[i]; }
-      if (last) {
-        // the child state, stored now so no register holds it through the loop
+      if (surv) {
         dst->s[lane][0] = cs0;
         dst->s[lane][1] = cs1;
-#pragma unroll
-        for (int i = 2; i < N; i++) dst->s[lane][i] = fs[i];
       }
+#pragma unroll
+      for (int i = 2; i < N; i++) {
+        const double f = __shfl_sync(hm, S[i], pp, LPJ);
+        if (surv) dst->s[lane][i] = f;
+      }
+    }
+    path = shfl64<LPJ>(q, pp, hm) | (unsigned long long)hh;
+    const unsigned pn = __shfl_sync(hm, (unsigned)perm | ((unsigned)new_next << 5), pp, LPJ);
+    perm = (int)(pn & 31u);
+    nxt = (int)(pn >> 5);
+    cur = __shfl_sync(hm, cur, pp, LPJ);
+    cur = (cur & ~(1u << (pos & 31))) | ((uint32_t)hh << (pos & 31));
+    if (surv) {
       cost = __dsub_rn(__longlong_as_double(Lk), min_cost);
-      path = npath;
-      nxt = nnext;
       slot = Ls;
+      if (links_matter) sm.key[nb][Ls] = key_of(cost);
+    }
+    if (cross) {
+      // the word is complete: bring the ring's words to their lanes, and enter
+      // the next one
 #pragma unroll
       for (int w = 0; w < RW; w++) {
-        uint32_t v = reg_word<RW>(nring[w]);
-        if (w == (pos >> 5)) v = (v & ~(1u << (pos & 31))) | ((uint32_t)hh << (pos & 31));
-        ring[w] = v;
+        uint32_t r = reg_word<RW>(ring[w]);
+        if (w < W) r = __shfl_sync(hm, r, perm, LPJ);
+        if (w == (pos >> 5)) r = cur;
+        ring[w] = r;
       }
-      sm.key[nb][Ls] = key_of(cost);
+      perm = lane;
+#pragma unroll
+      for (int w = 0; w < RW; w++) {
+        const uint32_t r = reg_word<RW>(ring[w]);
+        if (w == (next_pos >> 5)) cur = r;
+      }
     }
     __syncwarp(hm);
     if (n_new < n_old) { c_conv++; c_coll++; }
@@ -674,6 +906,13 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     err = __reduce_max_sync(hm, err);
     if (err && lane == 0) atomicMax(status, err);
     return;
+  }
+#pragma unroll
+  for (int w = 0; w < RW; w++) {
+    uint32_t r = reg_word<RW>(ring[w]);
+    if (w < W) r = __shfl_sync(hm, r, perm, LPJ);
+    if (w == (pos >> 5)) r = cur;
+    ring[w] = r;
   }
   if (lane < n) {
     dst->cost[lane] = cost;
@@ -708,9 +947,10 @@ template <int N, int LPJ>
 __global__ void __launch_bounds__(32, LPJ == 32 ? 13 : 10)
 sdm_jobs_kernel(SdmParams P, const SdmJob* __restrict__ jobs, int njobs,
                 int* __restrict__ job_counter, SdmCtx* __restrict__ ctxs,
-                int* __restrict__ status) {
+                int* __restrict__ status, int groups) {
   extern __shared__ __align__(16) unsigned char sdm_smem_raw[];
   const int wl = threadIdx.x & 31;
+  if (wl / LPJ >= groups) return;   // jobs per warp of this launch
   const int lane = wl & (LPJ - 1);
   const unsigned hm = job_mask<LPJ>(wl - lane);
   WarpSmem<LPJ>& sm =
@@ -925,13 +1165,14 @@ static int launch_wide(const SdmParams& P, dim3 grid, const SdmJob* d_jobs, int 
 
 template <int LPJ>
 static int launch_lpj(const SdmParams& P, dim3 grid, const SdmJob* d_jobs, int njobs,
-                      int* d_counter, SdmCtx* d_ctxs, int* d_status, cudaStream_t stream) {
-  const size_t smem = sizeof(WarpSmem<LPJ>) * (size_t)(32 / LPJ);
+                      int* d_counter, SdmCtx* d_ctxs, int* d_status, int groups,
+                      cudaStream_t stream) {
+  const size_t smem = sizeof(WarpSmem<LPJ>) * (size_t)groups;
   switch (P.order) {
 #define DSD_CASE(NN)                                                                       \
   case NN:                                                                                 \
     sdm_jobs_kernel<NN, LPJ><<<grid, 32, smem, stream>>>(P, d_jobs, njobs, d_counter, d_ctxs, \
-                                                         d_status);                        \
+                                                         d_status, groups);                \
     break;
     DSD_CASE(2) DSD_CASE(3) DSD_CASE(4) DSD_CASE(5) DSD_CASE(6)
     DSD_CASE(7) DSD_CASE(8) DSD_CASE(9) DSD_CASE(10)
@@ -971,8 +1212,9 @@ int launch_sdm_jobs(const SdmParams& P, const SdmJob* d_jobs, int njobs, int* d_
       return launch_sdm_scalar(P, d_jobs, njobs, d_ctxs, stream);
     }
   }
-  const int lanes = launch_lanes(P, njobs, max_blocks);
-  const int jpc = 32 / lanes;
+  int groups = 1;
+  const int lanes = launch_lanes(P, njobs, max_blocks, &groups);
+  const int jpc = groups;
   int blocks = (njobs + jpc - 1) / jpc;
   if (max_blocks > 0 && blocks > max_blocks) blocks = max_blocks;
   cudaMemsetAsync(d_counter, 0, sizeof(int), stream);
@@ -986,11 +1228,11 @@ int launch_sdm_jobs(const SdmParams& P, const SdmJob* d_jobs, int njobs, int* d_
   }
   note_kernel("sdm_jobs_kernel", P.order, lanes);
   switch (lanes) {
-    case 32: rc = launch_lpj<32>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, stream); break;
-    case 16: rc = launch_lpj<16>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, stream); break;
-    case 8: rc = launch_lpj<8>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, stream); break;
-    case 4: rc = launch_lpj<4>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, stream); break;
-    default: rc = launch_lpj<2>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, stream); break;
+    case 32: rc = launch_lpj<32>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    case 16: rc = launch_lpj<16>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    case 8: rc = launch_lpj<8>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    case 4: rc = launch_lpj<4>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    default: rc = launch_lpj<2>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
   }
   if (rc) return rc;
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
