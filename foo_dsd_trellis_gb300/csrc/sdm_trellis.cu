@@ -29,6 +29,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdio>
 
 namespace dsdgpu {
@@ -115,6 +116,31 @@ __host__ __device__ constexpr int mid_g_at(int k) {
   return 2;
 }
 
+// FP64 operations that stay under the branch they are written under, and the
+// count of that branch's passes (0 or 1): a loop stays a branch, while a short
+// condition becomes a predicate, under which an FP64 instruction costs its 64
+// cycles whether its result is wanted or not (measured).
+__device__ __forceinline__ double vmul(double a, double b) {
+  double r;
+  asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+__device__ __forceinline__ double vadd(double a, double b) {
+  double r;
+  asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+__device__ __forceinline__ double vsub(double a, double b) {
+  double r;
+  asm volatile("sub.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+__device__ __forceinline__ int all_products(bool zg) {
+  int z = zg ? 0 : 1;
+  asm volatile("" : "+r"(z));
+  return z;
+}
+
 // Operation k of the shared part, inputs S[1..N-1] (a child's state), into
 // np (with scratch tg).  Orders respect the dependencies when k runs
 // 0, 1, 2, ...
@@ -141,13 +167,16 @@ __device__ __forceinline__ void shared_op(int k, const SdmParams& P, const doubl
   k -= 1;
   if (k < Z) { const int i = mid_g_at<N>(k); np.D[i] = __dsub_rn(np.D[i], tg[i]); return; }
   k -= Z;
-  if (k == 0 && !zg) {
+  if (k == 0) {
     // the products with the g that are zero in the table's filters
-    if (g_zero<N>(0)) np.G0 = __dmul_rn(P.g[0], S[1]);
-    else np.G1 = __dmul_rn(P.g[1], S[2]);
+#pragma unroll 1
+    for (int z = all_products(zg); __builtin_expect(z > 0, 0); z--) {
+      if (g_zero<N>(0)) np.G0 = vmul(P.g[0], S[1]);
+      else np.G1 = vmul(P.g[1], S[2]);
 #pragma unroll
-    for (int i = 2; i <= N - 2; i++)
-      if (g_zero<N>(i)) np.D[i] = __dsub_rn(np.D[i], __dmul_rn(P.g[i], S[i + 1]));
+      for (int i = 2; i <= N - 2; i++)
+        if (g_zero<N>(i)) np.D[i] = vsub(np.D[i], vmul(P.g[i], S[i + 1]));
+    }
   }
   if (k < N - 2) { const int i = 2 + k; np.A[i] = __dmul_rn(P.a[i], np.D[i]); return; }
 }
@@ -471,9 +500,13 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     const unsigned long long q = (path << 1) & mask;
     double S[N];          // the children's shared state s[1..N-1] (clamped)
     S[0] = 0.0;
-    const double d0 = __dadd_rn(g_zero<N>(0) && zg ? cs0 : __dsub_rn(cs0, pk.G0), x);
+    double d0 = __dadd_rn(g_zero<N>(0) ? cs0 : __dsub_rn(cs0, pk.G0), x);
     double d1 = __dadd_rn(cs1, cs0);
-    if (N >= 3 && !(g_zero<N>(1) && zg)) d1 = __dsub_rn(d1, pk.G1);
+    if (N >= 3 && !g_zero<N>(1)) d1 = __dsub_rn(d1, pk.G1);
+    for (int z = all_products(zg); __builtin_expect(z > 0, 0); z--) {
+      if (g_zero<N>(0)) d0 = vadd(vsub(cs0, pk.G0), x);
+      else if (N >= 3) d1 = vsub(d1, pk.G1);
+    }
     double v = __dadd_rn(x, __dmul_rn(P.a[0], d0));
     v = __dadd_rn(v, __dmul_rn(P.a[1], d1));
 
@@ -1185,29 +1218,85 @@ static int launch_lpj(const SdmParams& P, dim3 grid, const SdmJob* d_jobs, int n
 bool sdm_scalar_eligible(const SdmParams& P, int max_blocks);   // sdm_scalar.cu
 int launch_sdm_scalar(const SdmParams& P, const SdmJob* d_jobs, int njobs, SdmCtx* d_ctxs,
                       cudaStream_t stream);
-int sdm_split_jobs_per_warp(const SdmParams& P);                 // sdm_split.cu
-bool sdm_split_supported(const SdmParams& P);
-int launch_sdm_split(const SdmParams& P, const SdmJob* d_jobs, int njobs, SdmCtx* d_ctxs,
-                     cudaStream_t stream);
+int launch_sdm_child_small(const SdmParams& P, int lanes, const SdmJob* d_jobs, int njobs,
+                           SdmCtx* d_ctxs, int* d_status, cudaStream_t stream);   // sdm_child_small.cu
+int launch_sdm_child_large(const SdmParams& P, int lanes, const SdmJob* d_jobs, int njobs,
+                           SdmCtx* d_ctxs, int* d_status, cudaStream_t stream);   // sdm_child_large.cu
 
-// Host-side launcher: each warp-sized CTA runs 32 / LPJ jobs side by side
-// (lanes_per_job); max_blocks caps the CTAs.  Uncapped launches of small
-// trellises take their own kernels: while the jobs fit in two warps per
-// scheduler, each candidate's NTF advance spread over lanes (sdm_split.cu,
-// K <= 2, or K <= 4 up to order 8: the shortest step); beyond that, at
-// K <= 2, one job per thread (sdm_scalar.cu, the fewest FP64 instructions per
-// job).
+// FP64 instructions of a step of the child kernel with H lanes a child: per
+// component of a lane the product with g (where a lane has one that is not
+// structurally zero), the two sums and the product with a; v; and e, its
+// square, the cost, s_0 and the cost's normalisation.
+static int child_ops(int N, int H) {
+  const int C = (N + H - 1) / H;
+  int m = 0, d = 1;
+  for (int j = 0; j < C; j++) {
+    bool need = false;
+    for (int q = 0; q < H; q++) {
+      const int i = q * C + j;
+      if (i <= N - 2 && (i & 1) != ((N & 1) ? 0 : 1)) need = true;
+    }
+    m += need;
+    d += need && j > 0;
+  }
+  return m + C + d + C + N + 5;
+}
+
+// Lanes of the child kernel (sdm_child.h) for a launch of njobs jobs without a
+// block cap, or 0 for the other kernels.  With w warps a scheduler a step takes
+// about 66 cycles an FP64 instruction and 800 more (w <= 1), or 76 w cycles an
+// FP64 instruction (the FP64 unit is the SM's: 19 cycles a warp instruction)
+// and 650 more; fewer lanes a job are more instructions a step over fewer
+// warps.  Measured cycles a step at order 6, by lanes a job:
+//   K = 2:  430 jobs 1,630 / 1,873 / 2,379 / 2,748 at 32 / 16 / 8 / 4 lanes,
+//           1,722 jobs 4,241 / 2,571 / 2,628 / 3,011
+//   K = 4:  608 jobs 1,887 / 2,565 / 2,935 at 32 / 16 / 8, 1,216 jobs 3,162 / 2,790 / 3,040
+//   K = 8:  608 jobs 2,504 / 3,215 at 32 / 16, 1,216 jobs 4,414 / 3,393
+// The warp kernel's step (one candidate a lane, its selection in sequence with
+// its arithmetic) takes 5,500 cycles alone and 8,925 at order 8 with 2.47 warps
+// a scheduler (the child kernel 7,600); the per-thread kernel (K <= 2) 9,600.
+static int child_lanes(const SdmParams& P, int njobs) {
+  const int K = P.cands, N = P.order;
+  if (K > 16) return 0;
+  const double pipes = 4.0 * (resident_warps() / 16);
+  auto warps = [&](int jpw) { return (double)((njobs + jpw - 1) / jpw) / pipes; };
+  const int KC = K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+  int best = 0;
+  double cost = 1e300;
+  for (int lanes = 32; lanes >= 2 * KC; lanes >>= 1) {
+    const double ops = child_ops(N, lanes / (2 * KC)), w = warps(32 / lanes);
+    const double c = std::max(66.0 * ops + 800.0, 76.0 * ops * w + 650.0);
+    if (c < cost) { cost = c; best = lanes; }
+  }
+  double other = 1e300;
+  if (K <= 2) {
+    other = std::max(9600.0, 76.0 * K * (5.0 * N + 6.0) * warps(32));
+  } else if (K > 4 && P.lat <= 32 * kRegRingWords) {
+    const int lanes = min_lanes(K);
+    const double slots = pipes / 4.0 * 10.0;
+    const int groups = (int)std::min(32.0 / lanes, std::max(1.0, std::ceil(njobs / slots)));
+    other = std::max(5500.0, 89.0 * 5.0 * N * warps(groups));
+  }
+  return other < cost ? 0 : best;
+}
+
+// Host-side launcher: each warp-sized CTA of the warp kernel runs 32 / LPJ
+// jobs side by side (lanes_per_job); max_blocks caps the CTAs.  Uncapped
+// launches at K <= 16 take the child kernel by the rule above, and at K <= 2
+// with more jobs than that serves the per-thread kernel (sdm_scalar.cu, the
+// fewest FP64 instructions per job).
 int launch_sdm_jobs(const SdmParams& P, const SdmJob* d_jobs, int njobs, int* d_counter,
                     SdmCtx* d_ctxs, int* d_status, int max_blocks, cudaStream_t stream) {
   if (njobs <= 0) return 0;
-  if (P.lanes == 0 && max_blocks == 0 && P.lat <= 32 * kRegRingWords) {
-    const long long split_cap = (long long)sdm_split_jobs_per_warp(P) * 2 * 4 * (resident_warps() / 16);
-    if (sdm_split_supported(P) && njobs <= split_cap) {
-      if (P.order <= 8) note_kernel("sdm_split_kernel", P.order, 8, P.cands <= 2 ? 2 : 4);
-      else note_kernel("sdm_split_kernel", P.order, 16, 2);
-      return launch_sdm_split(P, d_jobs, njobs, d_ctxs, stream);
+  if (P.lanes == 0 && max_blocks == 0) {
+    const int cl = child_lanes(P, njobs);
+    if (cl > 0) {
+      const int KC = P.cands <= 2 ? 2 : P.cands <= 4 ? 4 : P.cands <= 8 ? 8 : 16;
+      note_kernel("sdm_child_kernel", P.order, KC, cl / (2 * KC));
+      return KC <= 4 ? launch_sdm_child_small(P, cl, d_jobs, njobs, d_ctxs, d_status, stream)
+                     : launch_sdm_child_large(P, cl, d_jobs, njobs, d_ctxs, d_status, stream);
     }
-    if (sdm_scalar_eligible(P, max_blocks)) {
+    if (P.lat <= 32 * kRegRingWords && sdm_scalar_eligible(P, max_blocks)) {
       note_kernel("sdm_scalar_kernel", P.order);
       return launch_sdm_scalar(P, d_jobs, njobs, d_ctxs, stream);
     }

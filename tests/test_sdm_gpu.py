@@ -437,3 +437,65 @@ def test_state_distance(oracle):
     assert d.value == 0.0
     assert sdm.L.dsdgpu_sdm_state_distance(sdm.h, 0, 2, C.byref(d)) == _lib.ERR_ARG
     sdm.close()
+
+
+@pytest.mark.parametrize("K,depth,lat", [(32, 64, 128), (32, 6, 33), (17, 3, 64), (16, 48, 31),
+                                         (9, 32, 300), (8, 4, 256), (5, 3, 32), (4, 2, 65),
+                                         (2, 1, 1)])
+def test_costs_the_sort_words_do_not_tell(oracle, K, depth, lat):
+    """Costs that the selection's 32-bit words leave undecided take its whole
+    comparison: silence (equal costs from the first sample), a level far below
+    and far above the words' range, and equal paths on most samples (short path
+    masks), in blocks that end inside and at the ring's words."""
+    f = _ntf("clans-7" if K > 8 else "clans-6", 5644800)
+    x = np.concatenate([np.zeros(400), 1e-9 * multitone(300, seed=K), 0.5 * multitone(700, seed=K + 1),
+                        np.array([1e4, -1e60, 1e120]), 0.3 * multitone(600, seed=K + 2)])
+    ref = _ora(oracle, f, depth, K, lat)
+    g = _gpu_sdm(f, depth, K, lat)
+    for lo, hi in ((0, 1), (1, 33), (33, 640), (640, len(x))):
+        got = g.process_block(torch.from_numpy(x[lo:hi].copy()).cuda())[0].cpu().numpy()
+        np.testing.assert_array_equal(got, oracle.sdm_bits(ref, x[lo:hi]))
+    info, q = ref.info(), g.query(0)
+    assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
+        (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"])
+    np.testing.assert_array_equal(q["best_state"], ref.best_state())
+
+
+@pytest.mark.parametrize("K,depth,lat,njobs,order", [
+    (2, 4, 40, 5, 6), (2, 4, 64, 900, 6), (2, 40, 9, 1900, 7), (1, 8, 33, 4000, 8),
+    (4, 8, 32, 7, 6), (3, 6, 31, 700, 5), (4, 50, 65, 1400, 8), (8, 4, 256, 3, 6),
+    (6, 16, 20, 700, 7), (7, 5, 32, 1300, 8), (16, 48, 32, 6, 8), (12, 5, 300, 9, 7)])
+def test_uneven_segments_share_warps(oracle, K, depth, lat, njobs, order):
+    """Small trellises put up to eight jobs on a warp, chosen by their number:
+    segments of uneven lengths around the 32-sample blocks (none, one and
+    many), with discards and seeds, each from a copied context, and the
+    contexts that they leave."""
+    from foo_dsd_trellis_gb300.sdm import SegmentSpec
+    f = _ntf({5: "sdm-5", 6: "clans-6", 7: "clans-7", 8: "clans-8"}[order], 5644800)
+    lens = [0, 1, 31, 32, 33, 63, 64, 65, 97, 400]
+    x = multitone(1200, seed=K + njobs) * 0.8
+    g = _gpu_sdm(f, depth, K, lat, nctx=njobs + 1)
+    base = _ora(oracle, f, depth, K, lat)
+    oracle.sdm_bits(base, x[:333])
+    g.process_block(torch.from_numpy(x[:333].copy()).cuda(), first=njobs)
+    seed = base.best_state() * 0.5
+    xs, sd = torch.from_numpy(x).cuda(), torch.from_numpy(seed).cuda()
+    specs = []
+    for i in range(njobs):
+        n, lo = lens[(i * 7 + i // 10) % len(lens)], 333 + i % 300
+        specs.append(SegmentSpec(xs[lo:lo + n], channel=i, discard=[0, 5, 40][i % 3], seed_from=njobs,
+                                 seed_state=sd if i % 2 and n else None))   # empty: a plain copy
+    outs = g.segments(specs)
+    for i in list(range(min(njobs, 24))) + list(range(24, njobs, 53)):
+        ctx = _ora(oracle, f, depth, K, lat)
+        ctx.copy_from(base)
+        n, lo = lens[(i * 7 + i // 10) % len(lens)], 333 + i % 300
+        if i % 2 and n:
+            ctx.seed(seed)
+        np.testing.assert_array_equal(outs[i].cpu().numpy(),
+                                      oracle.segment_bits(ctx, x[lo:lo + n], [0, 5, 40][i % 3]),
+                                      err_msg=str(i))
+        q, info = g.query(i), ctx.info()
+        assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
+            (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"]), i
+        np.testing.assert_array_equal(q["best_state"], ctx.best_state())
