@@ -40,6 +40,10 @@ int launch_pack_native(const uint8_t* bits, size_t stride, int nch, size_t n, ui
 struct dsdgpu_conv_state;   // UPOLS convolution (conv.cu)
 struct dsdgpu_decim_state;  // DSD -> PCM decimation (decim.cu)
 void decim_free(dsdgpu_decim_state* s);
+// DoP frames or decision bytes through the decimation chain (decim.cu)
+int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d_bits, size_t stride,
+              size_t count, float* d_pcm, size_t pcm_stride, double gain_start, double gain_end,
+              size_t* out_count);
 struct dsdgpu_lowpass_state;  // same-rate FIR lowpass (lowpass.cu)
 void lowpass_free(dsdgpu_lowpass_state* s);
 struct dsdgpu_precorr_state;  // PreCorr greedy SDM (precorr.cu)

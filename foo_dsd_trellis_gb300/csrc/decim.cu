@@ -2,12 +2,35 @@
 // (src/engine.c:566-577; chain src/fir.c:523-611 with 63-tap half-band /2
 // stages, ipp_downsample_d src/fir.c:467-487; gain ramp src/engine.c:879-889).
 //
-// Every stage is one launch, FP64, y[m] = sum_k h[k] x[2m - k] (the delay
-// line of the previous call stands in for negative indices), followed by a
-// small launch that keeps the stage's last 62 consumed inputs.  A stage
-// consumes floor(count / 2) * 2 inputs, as the reference's numIters =
-// in_count / factor.  IPP's summation order and use of FMA are not known, so
-// the stages take the cheapest exact-enough form:
+// Two forms:
+//
+// The whole chain at once (decim_mma_kernel).  All stages together are one
+// filter h of 62 (D - 1) + 1 taps and a decimation by D, over +-1 inputs: with
+// the inputs cut into blocks X[n] of B = max(D, 16), an output is
+//   y[n] = sum_j sum_r h[B j - r] X[n - j][r]
+// a matrix product with the taps on one side and decisions on the other.  The
+// taps are taken to 2^-55 of their scale or finer and cut into seven 8-bit
+// digits, which bf16 holds exactly; every partial sum is a whole number below
+// 2^24, so the tensor cores' FP32 accumulators are exact, and the digits' sums
+// are joined as 64-bit integers.  Only the taps' own rounding is left (an FP64
+// evaluation rounds every sum as well).  What bounds it: the tensor cores'
+// mma.sync rate (16 x 16 x 8 products, 448 multiply-adds an input decision).
+// The rows of a product tile are the 16 values of j modulo 16, the four groups
+// of j shift the columns, so that 16 (not 63) diagonals are left to add up.
+// The decisions are expanded in shared memory to byte selectors (one PRMT makes
+// two bf16 of two decisions; "no sample yet" selects zero), one 32-bit load a
+// fragment.  10 s of stereo DSD128 to 44.1 kHz: see kMmaMeasured below.
+//
+// The stages one by one, FP64, y[m] = sum_k h[k] x[2m - k] (the delay line of
+// the previous call stands in for negative indices), each followed by a small
+// launch that keeps the stage's last 62 consumed inputs.  A stage consumes
+// floor(count / 2) * 2 inputs, as the reference's numIters = in_count /
+// factor: a call whose length is not a multiple of D drops inputs at some
+// stage, and what follows is no longer one filter over the decisions.  The
+// next call's first outputs (those whose window reaches back over that point)
+// and calls shorter than 128 B then take this form; so do FP64 inputs.  IPP's
+// summation order and use of FMA are not known, so the stages take the
+// cheapest exact-enough form:
 //   * the 63-tap half-band's taps at odd k other than the centre are the
 //     design's zeros (|h| < 2e-17: they move an output by ~1e-17 of full scale), so
 //     only the 32 even taps and the centre tap are applied;
@@ -16,12 +39,15 @@
 //     8, each group's sum for every pattern of its 8 decisions is a table
 //     entry (4 x 256 FP64 values, sums in tap order), so an output is 4 table
 //     reads, the centre tap's +-h[31] and 4 adds.
-// The result differs from a tap-order sum of separately rounded products by
-// a few FP64 ulps (float32 output within 2e-7 of full scale).
+// Either form differs from a tap-order sum of separately rounded products by
+// at most a few FP64 ulps (float32 output within 2e-7 of full scale).
 #include "api_context.h"
 #include "fir_internal.h"
 
+#include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <vector>
 
 using namespace dsdgpu;
 
@@ -146,6 +172,248 @@ __global__ void decim_gain_f64_kernel(const double* __restrict__ y, size_t y_str
   out[(size_t)c * out_stride + t] = v;
 }
 
+// ---- the whole chain as one matrix product ----
+constexpr int kMmaDigits = 7;          // 8-bit digits of a tap
+constexpr int kMmaWarps = 7;
+constexpr int kMmaCols = 128;          // output blocks of a CTA
+constexpr int kMmaAcc = kMmaCols + 16; // product columns: 16 diagonals end in every output
+constexpr int kAccRow = kMmaAcc + 4;   // row of the product tile in shared memory
+
+struct MmaPlan {
+  int B;        // inputs a block
+  int F;        // outputs a block (1, or 16 / D below D = 16)
+  int T;        // groups of 16 lags
+  int shift;    // taps are integers over 2^shift
+};
+
+// One DoP float's 16 decisions: round(f * 2^23) half away from zero, low 16
+// bits (dop_unpack_kernel's FP64 expression; f * 2^23 is exact in FP32, and
+// below 2^23 its fraction too).
+__device__ __forceinline__ unsigned dop_word(float f) {
+  const float y = f * 8388608.0f;
+  int v = __float2int_rz(y);
+  if (fabsf(y) < 8388608.0f) {
+    const float fr = y - (float)v;
+    if (fr >= 0.5f) v++;
+    else if (fr <= -0.5f) v--;
+  }
+  return (unsigned)v & 0xffffu;
+}
+
+// Byte selectors (PRMT) out of 0x00BF3F80: bf16 +1 = 3F80, -1 = BF80, none = 0.
+constexpr unsigned kPool = 0x00bf3f80u;
+constexpr unsigned kSelNone = 0x33333333u;
+__device__ __forceinline__ unsigned sel4(unsigned w, int c) {
+  // decisions 2c, 2c+1 (low half) and 2c+8, 2c+9 of a word, MSB first
+  const unsigned t = w >> (6 - 2 * c);
+  const unsigned a = (t >> 9) & 1u, b = (t >> 8) & 1u, e = (t >> 1) & 1u, f = t & 1u;
+  return 0x20202020u - ((a << 4) | (b << 12) | (e << 20) | (f << 28));
+}
+
+struct MmaIn {
+  const float* dop;        // DoP frames (kDop) or decision bytes
+  const uint8_t* bits;
+  size_t stride;
+  long long count;         // decisions of this call
+  const uint8_t* tail;     // decisions before it, newest last, tail_len of them (nullptr: none)
+  int tail_len;
+  size_t tail_stride;
+};
+
+// decision `i` of the stream: 0, 1, or 2 for none
+template <bool kDop>
+__device__ __forceinline__ unsigned decision(const MmaIn& I, int c, long long i) {
+  if (i < 0) {
+    const long long k = i + I.tail_len;
+    return k >= 0 ? I.tail[(size_t)c * I.tail_stride + k] : 2u;
+  }
+  if (i >= I.count) return 2u;
+  if (kDop) return (dop_word(I.dop[(size_t)c * I.stride + (i >> 4)]) >> (15 - (int)(i & 15))) & 1u;
+  return I.bits[(size_t)c * I.stride + i] & 1u;
+}
+
+template <bool kDop>
+__global__ void __launch_bounds__(32 * kMmaWarps)
+decim_mma_kernel(const MmaPlan M, const MmaIn I, const uint4* __restrict__ taps, int col_first,
+                 unsigned col_tiles, unsigned per_ch, long long n_out, double scale, double g_start, double g_step,
+                 int apply, float* __restrict__ out, size_t out_stride,
+                 uint8_t* __restrict__ new_tail, int keep, long long total) {
+  extern __shared__ __align__(16) unsigned mma_smem[];
+  const int c = (int)(blockIdx.x / per_ch);
+  const unsigned bx = blockIdx.x - (unsigned)c * per_ch;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (bx >= col_tiles) {
+    // the decisions the next call looks back to: the last `keep` of (tail ++ input)
+    const int part = (int)(bx - col_tiles), parts = (int)(per_ch - col_tiles);
+    for (int k = part * (int)blockDim.x + tid; k < keep; k += parts * (int)blockDim.x)
+      new_tail[(size_t)c * I.tail_stride + k] =
+          (uint8_t)decision<kDop>(I, c, total - keep + k - I.tail_len);
+    return;
+  }
+  const int KS = M.B >> 4;                       // 16-decision steps of a block
+  const int pitch = 4 * KS + 4;                  // words of a column (its lanes on distinct banks)
+  const long long n0 = col_first + (long long)bx * kMmaCols;
+  const int cols = kMmaCols + 16 * M.T;          // columns n0 - 16 T .. n0 + 127
+  for (int k = tid; k < cols * KS; k += blockDim.x) {
+    const int col = k / KS, ks = k % KS;
+    const long long i = (n0 - 16 * M.T + col) * M.B + 16 * ks;
+    unsigned w = 0u;
+    uint4 sel;
+    if (i >= 0 && i + 16 <= I.count) {
+      if (kDop) {
+        w = dop_word(I.dop[(size_t)c * I.stride + (i >> 4)]);
+      } else {
+        const uint8_t* b = I.bits + (size_t)c * I.stride + i;
+#pragma unroll
+        for (int u = 0; u < 16; u++) w |= (unsigned)(b[u] & 1u) << (15 - u);
+      }
+      sel = make_uint4(sel4(w, 0), sel4(w, 1), sel4(w, 2), sel4(w, 3));
+    } else {
+      unsigned none = 0u;
+      for (int u = 0; u < 16; u++) {
+        const unsigned d = decision<kDop>(I, c, i + u);
+        w |= (d & 1u) << (15 - u);
+        none |= (d >> 1) << (15 - u);
+      }
+      auto with = [&](int q) {
+        const unsigned t = none >> (6 - 2 * q);
+        const unsigned a = (t >> 9) & 1u, b = (t >> 8) & 1u, e = (t >> 1) & 1u, f = t & 1u;
+        const unsigned m = (a * 0x000000ffu) | (b * 0x0000ff00u) | (e * 0x00ff0000u) | (f * 0xff000000u);
+        return (sel4(w, q) & ~m) | (kSelNone & m);
+      };
+      sel = make_uint4(with(0), with(1), with(2), with(3));
+    }
+    *reinterpret_cast<uint4*>(&mma_smem[col * pitch + 4 * ks]) = sel;
+  }
+  __syncthreads();
+  // product tiles: one digit of one output phase a warp at a time
+  const int groups = kMmaDigits * M.F;
+  const int steps = M.T * KS;
+  for (int g0 = 0; g0 < groups; g0 += kMmaWarps) {
+    const int g = g0 + warp;                     // (phase, digit)
+    float acc[kMmaAcc / 8][4];
+#pragma unroll
+    for (int n = 0; n < kMmaAcc / 8; n++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) acc[n][r] = 0.0f;
+    const uint4* A = taps + ((size_t)g * steps) * 32 + lane;
+    uint4 an = A[0];
+    const unsigned* sb = mma_smem + (lane >> 2) * pitch + (lane & 3);
+    for (int st = 0; st < steps; st++) {
+      const uint4 a = an;
+      if (st + 1 < steps) an = A[(size_t)(st + 1) * 32];
+      const int t = st / KS, ks = st - t * KS;
+      const unsigned* col = sb + 16 * (M.T - 1 - t) * pitch + 4 * ks;
+#pragma unroll
+      for (int n = 0; n < kMmaAcc / 8; n++) {
+        const unsigned sel = col[8 * n * pitch];
+        const unsigned b0 = __byte_perm(kPool, 0u, sel), b1 = __byte_perm(kPool, 0u, sel >> 16);
+        asm volatile(
+            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+            "{%8,%9}, {%0,%1,%2,%3};"
+            : "+f"(acc[n][0]), "+f"(acc[n][1]), "+f"(acc[n][2]), "+f"(acc[n][3])
+            : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
+      }
+    }
+    // the diagonals: y[n] = sum_i acc[i][n - i], whole numbers below 2^24.
+    // The tiles lie behind the selectors, which further phases still read.
+    float* tile = reinterpret_cast<float*>(mma_smem + cols * pitch) + warp * 16 * kAccRow;
+    int* sums = reinterpret_cast<int*>(mma_smem + cols * pitch) + kMmaWarps * 16 * kAccRow;
+#pragma unroll
+    for (int n = 0; n < kMmaAcc / 8; n++) {
+      float* p = tile + (lane >> 2) * kAccRow + 8 * n + 2 * (lane & 3);
+      *reinterpret_cast<float2*>(p) = make_float2(acc[n][0], acc[n][1]);
+      *reinterpret_cast<float2*>(p + 8 * kAccRow) = make_float2(acc[n][2], acc[n][3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int n = 0; n < kMmaCols / 32; n++) {
+      float y = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 16; i++) y += tile[i * kAccRow + 16 + 32 * n + lane - i];
+      sums[warp * kMmaCols + 32 * n + lane] = (int)y;
+    }
+    __syncthreads();
+    // groups of one round are the digits of one phase, in the warps' order
+    if (tid < kMmaCols) {
+      const long long m = (n0 + tid) * M.F + g0 / kMmaWarps;
+      if (m < n_out) {
+        long long y = 0;
+#pragma unroll
+        for (int k = 0; k < kMmaDigits; k++) y += (long long)sums[k * kMmaCols + tid] << (8 * k);
+        double v = __dmul_rn((double)y, scale);
+        if (apply) v = __dmul_rn(v, __dadd_rn(g_start, __dmul_rn(g_step, (double)m)));
+        out[(size_t)c * out_stride + m] = (float)v;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+__host__ size_t mma_smem_bytes(const MmaPlan& M) {
+  return sizeof(unsigned) * (size_t)(kMmaCols + 16 * M.T) * (4 * (M.B >> 4) + 4) +
+         sizeof(float) * (size_t)kMmaWarps * 16 * kAccRow + sizeof(int) * kMmaWarps * kMmaCols;
+}
+
+// The plan of `stages` stages and its taps in the order of the A fragments:
+// [phase][digit][16-lag group][step][lane][4 registers of two bf16].
+std::vector<uint32_t> mma_taps(int stages, const DecNz& nz, MmaPlan* M) {
+  const int D = 1 << stages;
+  M->B = D < 16 ? 16 : D;
+  M->F = M->B / D;
+  // the stages' combined response: stage k's taps 2^k inputs apart
+  std::vector<double> h(1, 1.0);
+  for (int k = 0; k < stages; k++) {
+    const int gap = 1 << k;
+    std::vector<double> n(h.size() + (size_t)62 * gap, 0.0);
+    for (size_t i = 0; i < h.size(); i++)
+      for (int q = 0; q < kNzTaps; q++) n[i + (size_t)nz.k[q] * gap] += h[i] * nz.h[q];
+    h.swap(n);
+  }
+  const long long last = (long long)h.size() - 1;
+  const int J = (int)((last + M->B - 1) / M->B) + 1;
+  M->T = (J + 15) / 16;
+  double peak = 0.0;
+  for (double v : h) peak = std::max(peak, std::fabs(v));
+  M->shift = 61;
+  while (std::ldexp(peak, M->shift) > std::ldexp(1.0, 54)) M->shift--;
+  const int KS = M->B / 16, steps = M->T * KS;
+  std::vector<uint32_t> out((size_t)M->F * kMmaDigits * steps * 32 * 4, 0u);
+  auto bf16 = [](int v) {   // |v| <= 128: exact
+    float f = (float)v;
+    uint32_t u;
+    memcpy(&u, &f, 4);
+    return u >> 16;
+  };
+  std::vector<int8_t> dig(h.size() * kMmaDigits);
+  for (size_t i = 0; i < h.size(); i++) {
+    long long v = std::llrint(std::ldexp(h[i], M->shift));
+    for (int k = 0; k < kMmaDigits; k++) {   // balanced digits, -128 .. 127
+      int d = (int)(v & 255);
+      if (d > 127) d -= 256;
+      dig[i * kMmaDigits + k] = (int8_t)d;
+      v = (v - d) >> 8;
+    }
+  }
+  for (int ph = 0; ph < M->F; ph++)
+    for (int k = 0; k < kMmaDigits; k++)
+      for (int t = 0; t < M->T; t++)
+        for (int ks = 0; ks < KS; ks++)
+          for (int lane = 0; lane < 32; lane++)
+            for (int r = 0; r < 4; r++) {
+              uint32_t w = 0;
+              for (int e = 0; e < 2; e++) {
+                const int row = lane / 4 + (r & 1) * 8;
+                const int kk = 2 * (lane % 4) + e + (r >> 1) * 8;
+                const long long tap = (long long)D * ph + (long long)M->B * (16 * t + row) - (16 * ks + kk);
+                const int d = tap >= 0 && tap <= last ? dig[(size_t)tap * kMmaDigits + k] : 0;
+                w |= bf16(d) << (16 * e);
+              }
+              out[((((size_t)ph * kMmaDigits + k) * steps + (size_t)t * KS + ks) * 32 + lane) * 4 + r] = w;
+            }
+  return out;
+}
+
 unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -159,7 +427,21 @@ struct dsdgpu_decim_state {
   double* d_dly = nullptr;      // [stage][nch][62]
   double* d_buf = nullptr;      // ping-pong [2][nch][row]
   size_t row = 0;
+  // the whole-chain form: its plan, taps, and the decisions before the next
+  // call (two buffers in turn)
+  MmaPlan mma{};
+  uint4* d_taps = nullptr;
+  uint8_t* d_tail = nullptr;    // [2][nch][tail_cap]
+  int tail_cap = 0, tail_len = 0, tail_buf = 0;
+  // what the next call continues from: nothing yet, the decisions in the tail
+  // (`ragged`: their last call's length was not whole blocks), or the stages'
+  // delay lines
+  enum { kFresh, kTail, kLines } from = kFresh;
+  bool ragged = false;
+  uint8_t* tail() const { return d_tail + (size_t)tail_buf * nch * tail_cap; }
   ~dsdgpu_decim_state() {
+    if (d_taps) cudaFree(d_taps);
+    if (d_tail) cudaFree(d_tail);
     if (d_lut) cudaFree(d_lut);
     if (d_dly) cudaFree(d_dly);
     if (d_buf) cudaFree(d_buf);
@@ -209,6 +491,168 @@ int launch_decim_f64_fresh(const double* in, size_t in_stride, long long count, 
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
+namespace {
+
+int ensure_rows(dsdgpu_context_t* c, dsdgpu_decim_state* s, size_t count) {
+  const size_t row = ((count / 2 + 1) + 31) & ~(size_t)31;
+  if (s->row >= row) return DSDGPU_OK;
+  if (s->d_buf) cudaFree(s->d_buf);
+  s->d_buf = nullptr;
+  s->row = 0;
+  if (cudaMalloc(&s->d_buf, sizeof(double) * 2 * row * (size_t)s->nch) != cudaSuccess)
+    return c->cuda_fail(cudaGetLastError(), "decimation buffers");
+  s->row = row;
+  return DSDGPU_OK;
+}
+
+// `count` decisions through the stages and their delay lines; the last
+// stage's outputs in *y (rows of s->row), *m of them.
+int staged(dsdgpu_context_t* c, dsdgpu_decim_state* s, const uint8_t* d_bits, size_t bits_stride,
+           size_t count, const double** y, size_t* m_out) {
+  const int nch = s->nch;
+  cudaStream_t st = c->stream;
+  const int rc = ensure_rows(c, s, count);
+  if (rc) return rc;
+  double* buf[2] = {s->d_buf, s->d_buf + s->row * (size_t)nch};
+  size_t cur = count;
+  const double* in = nullptr;
+  for (int k = 0; k < s->stages; k++) {
+    const long long m = (long long)(cur / 2);
+    double* out = buf[k & 1];
+    double* dly = s->d_dly + (size_t)k * nch * (kDecTaps - 1);
+    if (m > 0) {
+      if (k == 0) {
+        decim_bits_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, s->d_lut, s->taps.h[kDecTaps / 2], d_bits,
+                                                            bits_stride, m, dly, out, s->row, nch);
+        decim_dly_kernel<true><<<nch, 64, 0, st>>>(d_bits, nullptr, bits_stride, 2 * m, dly, nch);
+      } else {
+        decim_stage_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, in, s->row, m, dly, out, s->row,
+                                                             nch);
+        decim_dly_kernel<false><<<nch, 64, 0, st>>>(nullptr, in, s->row, 2 * m, dly, nch);
+      }
+      c->launches += 2;
+    }
+    in = out;
+    cur = (size_t)m;
+  }
+  *y = in;
+  *m_out = cur;
+  return DSDGPU_OK;
+}
+
+// The stages' delay lines as the calls so far leave them: zero at a stream's
+// start, else the stages run over the tail from rest.  The tail starts on a
+// whole block and is 64 blocks long (or the whole stream), which is longer
+// than any line's window, so its last values are the same as in one run.
+int to_lines(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
+  if (s->from == dsdgpu_decim_state::kLines) return DSDGPU_OK;
+  cudaMemsetAsync(s->d_dly, 0, sizeof(double) * (size_t)s->stages * s->nch * (kDecTaps - 1), c->stream);
+  if (s->from == dsdgpu_decim_state::kTail && s->tail_len > 0) {
+    const double* y = nullptr;
+    size_t m = 0;
+    const int rc = staged(c, s, s->tail(), (size_t)s->tail_cap, (size_t)s->tail_len, &y, &m);
+    if (rc) return rc;
+  }
+  s->from = dsdgpu_decim_state::kLines;
+  return DSDGPU_OK;
+}
+
+}  // namespace
+
+// One call of the decimation from DoP frames (d_dop, rows of `stride` floats)
+// or decision bytes (d_bits): the route by what the stream continues from (see
+// the head of the file).  DoP frames that have to take the stages are unpacked
+// into the context's scratch memory by the caller's `unpack` buffer.
+int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d_bits, size_t stride,
+              size_t count, float* d_pcm, size_t pcm_stride, double gain_start, double gain_end,
+              size_t* out_count) {
+  if (!c) return DSDGPU_ERR_ARG;
+  dsdgpu_decim_state* s = c->decim;
+  if (!s) return c->fail(DSDGPU_ERR_STATE, "decimation not set up");
+  if (nch != s->nch) return c->fail(DSDGPU_ERR_ARG, "channel count differs from the setup");
+  size_t n = count;
+  for (int k = 0; k < s->stages; k++) n /= 2;
+  if (out_count) *out_count = n;
+  if (count < 2) return DSDGPU_OK;
+  if ((!d_bits && !d_dop) || !d_pcm) return c->fail(DSDGPU_ERR_ARG, "null buffer");
+  if (pcm_stride < n) return c->fail(DSDGPU_ERR_ARG, "output stride too small");
+  cudaSetDevice(c->device);
+  cudaStream_t st = c->stream;
+  // gain ramp of engine_process_fir_gain (src/engine.c:879-889), then float
+  double gs = gain_start;
+  if (gs == 0.0) gs = gain_end;
+  const int apply = (gs != 1.0 || gain_end != 1.0) ? 1 : 0;
+  const double step = n > 1 ? (gain_end - gs) / (double)(n - 1) : 0.0;
+
+  const MmaPlan& M = s->mma;
+  int col_first = 0;
+  if (s->from == dsdgpu_decim_state::kLines || s->ragged) {
+    int rc = to_lines(c, s);
+    if (rc) return rc;
+    s->ragged = false;
+    s->tail_len = 0;
+    const bool all = count < (size_t)128 * M.B;
+    const size_t part = all ? count : (size_t)64 * M.B;
+    const uint8_t* bits = d_bits;
+    size_t bstride = stride;
+    if (d_dop) {
+      bstride = (part + 255) & ~(size_t)255;
+      rc = c->ensure_scratch(bstride * (size_t)nch);
+      if (rc) return rc;
+      rc = dsdgpu_dop_unpack(c, nch, d_dop, stride, part / 16, (uint8_t*)c->d_scratch, bstride);
+      if (rc) return rc;
+      bits = (const uint8_t*)c->d_scratch;
+    }
+    const double* y = nullptr;
+    size_t m = 0;
+    rc = staged(c, s, bits, bstride, part, &y, &m);
+    if (rc) return rc;
+    if (m > 0) {
+      decim_gain_kernel<<<nb((long long)m * nch, 256), 256, 0, st>>>(y, s->row, (long long)m, nch, gs,
+                                                                   step, apply, d_pcm, pcm_stride);
+      c->launches++;
+    }
+    if (all) {
+      const cudaError_t e = cudaGetLastError();
+      return e == cudaSuccess ? DSDGPU_OK : c->cuda_fail(e, "decimation launch");
+    }
+    col_first = 64;   // the windows of the outputs from here on lie in this call
+  }
+  MmaIn I{};
+  I.dop = d_dop;
+  I.bits = d_bits;
+  I.stride = stride;
+  I.count = (long long)count;
+  I.tail = s->tail();
+  I.tail_len = s->tail_len;
+  I.tail_stride = (size_t)s->tail_cap;
+  const int rag = (int)(count % (size_t)M.B);
+  const long long total = (long long)s->tail_len + (long long)count;
+  const int keep = (int)std::min<long long>(total, 64ll * M.B + rag);
+  uint8_t* next = s->d_tail + (size_t)(s->tail_buf ^ 1) * nch * s->tail_cap;
+  const long long cols = ((long long)n + M.F - 1) / M.F - col_first;
+  const unsigned tiles = (unsigned)((std::max(cols, 0ll) + kMmaCols - 1) / kMmaCols);
+  const unsigned per = tiles + (unsigned)((keep + 4095) / 4096);
+  const dim3 grid(per * (unsigned)nch);
+  const size_t smem = mma_smem_bytes(M);
+  const double scale = std::ldexp(1.0, -M.shift);
+  if (d_dop)
+    decim_mma_kernel<true><<<grid, 32 * kMmaWarps, smem, st>>>(M, I, s->d_taps, col_first, tiles, per, (long long)n,
+                                                               scale, gs, step, apply, d_pcm, pcm_stride,
+                                                               next, keep, total);
+  else
+    decim_mma_kernel<false><<<grid, 32 * kMmaWarps, smem, st>>>(M, I, s->d_taps, col_first, tiles, per, (long long)n,
+                                                                scale, gs, step, apply, d_pcm, pcm_stride,
+                                                                next, keep, total);
+  c->launches++;
+  s->tail_buf ^= 1;
+  s->tail_len = keep;
+  s->ragged = rag != 0;
+  s->from = dsdgpu_decim_state::kTail;
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? DSDGPU_OK : c->cuda_fail(e, "decimation launch");
+}
+
 extern "C" {
 
 int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int nch) {
@@ -239,11 +683,22 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
       lut[g * 256 + p] = acc;
     }
   const size_t dbytes = sizeof(double) * (size_t)S * nch * (kDecTaps - 1);
-  if (cudaMalloc(&s->d_dly, dbytes) != cudaSuccess || cudaMalloc(&s->d_lut, sizeof lut) != cudaSuccess) {
+  const std::vector<uint32_t> taps = mma_taps(S, s->nz, &s->mma);
+  s->tail_cap = 65 * s->mma.B;
+  if (cudaMalloc(&s->d_dly, dbytes) != cudaSuccess || cudaMalloc(&s->d_lut, sizeof lut) != cudaSuccess ||
+      cudaMalloc(&s->d_taps, taps.size() * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&s->d_tail, (size_t)2 * nch * s->tail_cap) != cudaSuccess) {
     delete s;
     return c->cuda_fail(cudaGetLastError(), "decimation buffers");
   }
+  const int smem = (int)mma_smem_bytes(s->mma);
+  if (cudaFuncSetAttribute(decim_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(decim_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+    delete s;
+    return c->cuda_fail(cudaGetLastError(), "decimation kernel attributes");
+  }
   cudaMemcpyAsync(s->d_lut, lut, sizeof lut, cudaMemcpyHostToDevice, c->stream);
+  cudaMemcpyAsync(s->d_taps, taps.data(), taps.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
   cudaMemsetAsync(s->d_dly, 0, dbytes, c->stream);
   decim_free(c->decim);
   c->decim = s;
@@ -253,70 +708,18 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
 int dsdgpu_decim_reset(dsdgpu_context_t* c) {
   if (!c) return DSDGPU_ERR_ARG;
   if (!c->decim) return c->fail(DSDGPU_ERR_STATE, "decimation not set up");
-  cudaSetDevice(c->device);
-  dsdgpu_decim_state* s = c->decim;
-  cudaMemsetAsync(s->d_dly, 0, sizeof(double) * (size_t)s->stages * s->nch * (kDecTaps - 1), c->stream);
-  return c->check_status();
+  // nothing on the device has to change: the next call starts from no history
+  c->decim->from = dsdgpu_decim_state::kFresh;
+  c->decim->tail_len = 0;
+  c->decim->ragged = false;
+  return DSDGPU_OK;
 }
 
 int dsdgpu_decim_process_async(dsdgpu_context_t* c, int nch, const uint8_t* d_bits,
                                size_t bits_stride, size_t count, float* d_pcm, size_t pcm_stride,
                                double gain_start, double gain_end, size_t* out_count) {
-  if (!c) return DSDGPU_ERR_ARG;
-  dsdgpu_decim_state* s = c->decim;
-  if (!s) return c->fail(DSDGPU_ERR_STATE, "decimation not set up");
-  if (nch != s->nch) return c->fail(DSDGPU_ERR_ARG, "channel count differs from the setup");
-  size_t n = count;
-  for (int k = 0; k < s->stages; k++) n /= 2;
-  if (out_count) *out_count = n;
-  if (count < 2) return DSDGPU_OK;
-  if (!d_bits || !d_pcm) return c->fail(DSDGPU_ERR_ARG, "null buffer");
-  if (pcm_stride < n) return c->fail(DSDGPU_ERR_ARG, "output stride too small");
-  cudaSetDevice(c->device);
-  cudaStream_t st = c->stream;
-  const size_t row = ((count / 2 + 1) + 31) & ~(size_t)31;
-  if (s->row < row) {
-    if (s->d_buf) cudaFree(s->d_buf);
-    s->d_buf = nullptr;
-    s->row = 0;
-    if (cudaMalloc(&s->d_buf, sizeof(double) * 2 * row * (size_t)nch) != cudaSuccess)
-      return c->cuda_fail(cudaGetLastError(), "decimation buffers");
-    s->row = row;
-  }
-  double* buf[2] = {s->d_buf, s->d_buf + s->row * (size_t)nch};
-  size_t cur = count;
-  const double* in = nullptr;
-  for (int k = 0; k < s->stages; k++) {
-    const long long m = (long long)(cur / 2);
-    double* out = buf[k & 1];
-    double* dly = s->d_dly + (size_t)k * nch * (kDecTaps - 1);
-    if (m > 0) {
-      if (k == 0) {
-        decim_bits_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, s->d_lut, s->taps.h[kDecTaps / 2], d_bits,
-                                                            bits_stride, m, dly, out, s->row, nch);
-        decim_dly_kernel<true><<<nch, 64, 0, st>>>(d_bits, nullptr, bits_stride, 2 * m, dly, nch);
-      } else {
-        decim_stage_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, in, s->row, m, dly, out, s->row,
-                                                             nch);
-        decim_dly_kernel<false><<<nch, 64, 0, st>>>(nullptr, in, s->row, 2 * m, dly, nch);
-      }
-      c->launches += 2;
-    }
-    in = out;
-    cur = (size_t)m;
-  }
-  // gain ramp of engine_process_fir_gain (src/engine.c:879-889), then float
-  double gs = gain_start;
-  if (gs == 0.0) gs = gain_end;
-  const int apply = (gs != 1.0 || gain_end != 1.0) ? 1 : 0;
-  const double step = n > 1 ? (gain_end - gs) / (double)(n - 1) : 0.0;
-  if (n > 0) {
-    decim_gain_kernel<<<nb((long long)n * nch, 256), 256, 0, st>>>(in, s->row, (long long)n, nch, gs,
-                                                                 step, apply, d_pcm, pcm_stride);
-    c->launches++;
-  }
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? DSDGPU_OK : c->cuda_fail(e, "decimation launch");
+  return decim_run(c, nch, nullptr, d_bits, bits_stride, count, d_pcm, pcm_stride, gain_start,
+                   gain_end, out_count);
 }
 
 int dsdgpu_decim_process_f64_async(dsdgpu_context_t* c, int nch, const double* d_in,
@@ -336,15 +739,12 @@ int dsdgpu_decim_process_f64_async(dsdgpu_context_t* c, int nch, const double* d
     return c->fail(DSDGPU_ERR_ARG, "row stride shorter than the count");
   cudaSetDevice(c->device);
   cudaStream_t st = c->stream;
-  const size_t row = ((count / 2 + 1) + 31) & ~(size_t)31;
-  if (s->row < row) {
-    if (s->d_buf) cudaFree(s->d_buf);
-    s->d_buf = nullptr;
-    s->row = 0;
-    if (cudaMalloc(&s->d_buf, sizeof(double) * 2 * row * (size_t)nch) != cudaSuccess)
-      return c->cuda_fail(cudaGetLastError(), "decimation buffers");
-    s->row = row;
-  }
+  int rc = to_lines(c, s);
+  if (rc) return rc;
+  s->ragged = false;
+  s->tail_len = 0;
+  rc = ensure_rows(c, s, count);
+  if (rc) return rc;
   double* buf[2] = {s->d_buf, s->d_buf + s->row * (size_t)nch};
   size_t cur = count;
   const double* in = d_in;

@@ -134,18 +134,11 @@ int dsdgpu_pipeline_process(dsdgpu_context_t* c, const float* d_pcm, size_t pcm_
   cudaSetDevice(c->device);
   const int nch = c->pipe_nch;
   if (c->pipe_pcm_out) {
-    // DSD -> PCM: DoP unpack into decision bytes, decimation to float rows
-    const size_t n_in = 16 * frames;
-    const size_t bit_row = (n_in + 255) & ~(size_t)255;
-    int rc = c->ensure_scratch(bit_row * (size_t)nch + 256);
-    if (rc) return rc;
-    uint8_t* d_bits = (uint8_t*)c->d_scratch;
+    // DSD -> PCM: DoP frames straight into the decimation, float rows out
     cudaEventRecord(c->ev[0], c->stream);
-    rc = dsdgpu_dop_unpack(c, nch, d_pcm, pcm_stride, frames, d_bits, bit_row);
-    if (rc) return rc;
     size_t n = 0;
-    rc = dsdgpu_decim_process_async(c, nch, d_bits, bit_row, n_in, (float*)d_out, out_stride,
-                                    gain_start, gain_end, &n);
+    int rc = decim_run(c, nch, d_pcm, nullptr, pcm_stride, 16 * frames, (float*)d_out, out_stride,
+                       gain_start, gain_end, &n);
     if (rc) return rc;
     cudaEventRecord(c->ev[5], c->stream);
     rc = c->check_status();

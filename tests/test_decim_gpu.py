@@ -90,3 +90,75 @@ def test_dsd_to_pcm_pipeline_sinad(oracle):
         s_got, s_ref = _sinad(got[c], fs_pcm, 997.0), _sinad(ref, fs_pcm, 997.0)
         assert abs(s_got - s_ref) < 0.01, (s_got, s_ref)
         assert s_got > 115.0, s_got
+
+
+@pytest.mark.parametrize("fs_in,fs_out", [(2822400, 1411200), (2822400, 705600), (2822400, 352800),
+                                          (2822400, 176400), (5644800, 44100), (11289600, 44100),
+                                          (22579200, 44100)])
+def test_decim_blocks_of_every_kind(oracle, fs_in, fs_out):
+    """Streams cut into calls that continue in each of the chain's forms: whole
+    blocks (one matrix product over the history), ragged ends (the next call
+    starts in the stages), calls of less than a block, calls around the 64 and
+    128 blocks where the forms change, and a reset; three channels whose rows
+    are wider than the call."""
+    from foo_dsd_trellis_gb300 import _lib
+    D = fs_in // fs_out
+    B = max(D, 16)
+    lens = [3 * B, 2 * B, 5, 200 * B + 7, 127 * B, 129 * B, 40 * B + 1, B - 1, 131 * B + B // 2,
+            64 * B, 300 * B]
+    if D == 512:
+        lens = lens[:8]
+    nch = 3
+    rng = np.random.default_rng(D)
+    L = _lib.load()
+    h = C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    _lib.check(h, L.dsdgpu_decim_setup(h, fs_in, fs_out, nch))
+    for rep in range(2):
+        refs = [oracle.Decimator(fs_in, fs_out) for _ in range(nch)]
+        for k, ln in enumerate(lens if rep == 0 else lens[:1] + lens[5:7]):
+            bits = (rng.random((nch, ln + 5)) > 0.4).astype(np.uint8)
+            blk = torch.from_numpy(bits).cuda()
+            out = torch.full((nch, ln // D + 3), 9.0, dtype=torch.float32, device="cuda")
+            m = C.c_size_t()
+            _lib.check(h, L.dsdgpu_decim_process(h, nch, C.c_void_p(blk.data_ptr()), blk.stride(0), ln,
+                                                 C.c_void_p(out.data_ptr()), out.stride(0), 1.0, 1.0,
+                                                 C.byref(m)))
+            got = out.cpu().numpy()
+            for c in range(nch):
+                want = refs[c].process(bits[c, :ln].astype(np.float64) * 2 - 1).astype(np.float32)
+                assert m.value == len(want), (k, ln)
+                np.testing.assert_allclose(got[c, : len(want)], want, rtol=0, atol=2e-7,
+                                           err_msg=f"call {k} of {ln}")
+                assert (got[c, len(want):] == 9.0).all()
+        _lib.check(h, L.dsdgpu_decim_reset(h))
+    L.dsdgpu_destroy(h)
+
+
+def test_decim_dop_equals_bits(oracle):
+    """The pipeline's DoP frames (read by the decimation itself) give what the
+    same decisions give as bytes: whole blocks, ragged ends and short calls."""
+    from foo_dsd_trellis_gb300 import _lib, ntf
+    from foo_dsd_trellis_gb300.pipeline import Encoder
+    fs_in, fs_out, nch = 5644800, 44100, 2
+    rng = np.random.default_rng(8)
+    enc = Encoder(fs_in, fs_out, nch, ntf.get_filter("clans-7", fs_in), 64, 32, 128,
+                  output_format=_lib.OUT_PCM)
+    L = _lib.load()
+    h = C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    _lib.check(h, L.dsdgpu_decim_setup(h, fs_in, fs_out, nch))
+    for frames in (8 * 40, 8 * 3, 3, 8 * 200 + 5, 8 * 500, 8 * 130, 1, 8 * 90):
+        bits = (rng.random((nch, 16 * frames)) > 0.5).astype(np.uint8)
+        dop = torch.from_numpy(np.stack([oracle.dop_float_frames(bits[c], 0) for c in range(nch)])).cuda()
+        a = torch.zeros((nch, frames // 8 + 4), dtype=torch.float32, device="cuda")
+        b = torch.zeros_like(a)
+        n, _ = enc.process(dop, a, 0.7, 0.9)
+        blk = torch.from_numpy(bits).cuda()
+        m = C.c_size_t()
+        _lib.check(h, L.dsdgpu_decim_process(h, nch, C.c_void_p(blk.data_ptr()), blk.stride(0),
+                                             16 * frames, C.c_void_p(b.data_ptr()), b.stride(0), 0.7, 0.9,
+                                             C.byref(m)))
+        assert n == m.value
+        assert torch.equal(a, b), frames
+    L.dsdgpu_destroy(h)
