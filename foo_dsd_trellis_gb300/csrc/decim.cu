@@ -13,13 +13,19 @@
 // digits, which bf16 holds exactly; every partial sum is a whole number below
 // 2^24, so the tensor cores' FP32 accumulators are exact, and the digits' sums
 // are joined as 64-bit integers.  Only the taps' own rounding is left (an FP64
-// evaluation rounds every sum as well).  What bounds it: the tensor cores'
-// mma.sync rate (16 x 16 x 8 products, 448 multiply-adds an input decision).
+// evaluation rounds every sum as well).
 // The rows of a product tile are the 16 values of j modulo 16, the four groups
 // of j shift the columns, so that 16 (not 63) diagonals are left to add up.
 // The decisions are expanded in shared memory to byte selectors (one PRMT makes
 // two bf16 of two decisions; "no sample yet" selects zero), one 32-bit load a
-// fragment.  10 s of stereo DSD128 to 44.1 kHz: see kMmaMeasured below.
+// fragment; a warp uses each fragment for two digits, since making it (three
+// half-rate integer instructions) takes as long as a product (mma.sync
+// m16n8k16: 8.35 cycles a scheduler, measured).  What bounds it: the tensor
+// pipe (active half of the time, ncu; 448 multiply-adds an input decision),
+// then the taps' loads from L2.  10 s of stereo DSD128 to 44.1 kHz, the whole
+// call: 4,571 us stage by stage, 357 us here (7 warps of one digit over all
+// columns 573, prmt by an intrinsic that masks its selector 577, one digit a
+// warp over half the columns 430, taps loaded a step ahead 428).
 //
 // The stages one by one, FP64, y[m] = sum_k h[k] x[2m - k] (the delay line of
 // the previous call stands in for negative indices), each followed by a small
@@ -174,7 +180,8 @@ __global__ void decim_gain_f64_kernel(const double* __restrict__ y, size_t y_str
 
 // ---- the whole chain as one matrix product ----
 constexpr int kMmaDigits = 7;          // 8-bit digits of a tap
-constexpr int kMmaWarps = 7;
+constexpr int kMmaParts = 3;           // a warp: two digits over a third of the columns
+constexpr int kMmaWarps = (kMmaDigits + 1) / 2 * kMmaParts;
 constexpr int kMmaCols = 128;          // output blocks of a CTA
 constexpr int kMmaAcc = kMmaCols + 16; // product columns: 16 diagonals end in every output
 constexpr int kAccRow = kMmaAcc + 4;   // row of the product tile in shared memory
@@ -203,11 +210,18 @@ __device__ __forceinline__ unsigned dop_word(float f) {
 // Byte selectors (PRMT) out of 0x00BF3F80: bf16 +1 = 3F80, -1 = BF80, none = 0.
 constexpr unsigned kPool = 0x00bf3f80u;
 constexpr unsigned kSelNone = 0x33333333u;
-__device__ __forceinline__ unsigned sel4(unsigned w, int c) {
-  // decisions 2c, 2c+1 (low half) and 2c+8, 2c+9 of a word, MSB first
-  const unsigned t = w >> (6 - 2 * c);
-  const unsigned a = (t >> 9) & 1u, b = (t >> 8) & 1u, e = (t >> 1) & 1u, f = t & 1u;
-  return 0x20202020u - ((a << 4) | (b << 12) | (e << 20) | (f << 28));
+// Selectors of lane c: decisions 2c, 2c+1 (low half) and 2c+8, 2c+9 of a word
+// whose bit k is decision k: bit 4 of bytes 0 .. 3, taken from 2 (-1) to 1 (+1).
+__device__ __forceinline__ unsigned sel4(unsigned wr, int c) {
+  const unsigned x = (wr << 4) >> (2 * c), y = (wr << 3) >> (2 * c);
+  return 0x20202020u - (__byte_perm(x, y, 0x5140) & 0x10101010u);
+}
+
+// two bf16 by the selector's low half (prmt's plain mode: nibbles 0 .. 3)
+__device__ __forceinline__ unsigned two(unsigned sel) {
+  unsigned r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(kPool), "r"(sel));
+  return r;
 }
 
 struct MmaIn {
@@ -232,8 +246,54 @@ __device__ __forceinline__ unsigned decision(const MmaIn& I, int c, long long i)
   return I.bits[(size_t)c * I.stride + i] & 1u;
 }
 
+// One warp's products: ND digits (16 rows each) by kN products of 8 columns,
+// over all steps, left in the digits' tiles in shared memory.
+constexpr int kN = kMmaAcc / 8 / kMmaParts;
+template <int ND>
+__device__ __forceinline__ void mma_tile(const uint4* __restrict__ A, int steps, int KS, int pitch,
+                                         const unsigned* sb, float* tile) {
+  float acc[ND][kN][4];
+#pragma unroll
+  for (int k = 0; k < ND; k++)
+#pragma unroll
+    for (int n = 0; n < kN; n++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) acc[k][n][r] = 0.0f;
+  const size_t digit = (size_t)steps * 32;
+  for (int t = steps / KS; t > 0; t--, sb -= 64) {   // the next 16 lags: 16 columns back
+    const unsigned* col = sb;
+#pragma unroll 4
+    for (int ks = 0; ks < KS; ks++, col += pitch, A += 32) {
+      uint4 a[ND];
+#pragma unroll
+      for (int k = 0; k < ND; k++) a[k] = A[k * digit];
+      unsigned sel[kN];
+#pragma unroll
+      for (int n = 0; n < kN; n++) sel[n] = col[32 * n];
+#pragma unroll
+      for (int n = 0; n < kN; n++) {
+        const unsigned b0 = two(sel[n]), b1 = two(sel[n] >> 16);
+#pragma unroll
+        for (int k = 0; k < ND; k++)
+          asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+              "{%8,%9}, {%0,%1,%2,%3};"
+              : "+f"(acc[k][n][0]), "+f"(acc[k][n][1]), "+f"(acc[k][n][2]), "+f"(acc[k][n][3])
+              : "r"(a[k].x), "r"(a[k].y), "r"(a[k].z), "r"(a[k].w), "r"(b0), "r"(b1));
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < ND; k++)
+#pragma unroll
+    for (int n = 0; n < kN; n++) {
+      float* p = tile + k * 16 * kAccRow + 8 * n;
+      *reinterpret_cast<float2*>(p) = make_float2(acc[k][n][0], acc[k][n][1]);
+      *reinterpret_cast<float2*>(p + 8 * kAccRow) = make_float2(acc[k][n][2], acc[k][n][3]);
+    }
+}
+
 template <bool kDop>
-__global__ void __launch_bounds__(32 * kMmaWarps)
+__global__ void __launch_bounds__(32 * kMmaWarps, 2)
 decim_mma_kernel(const MmaPlan M, const MmaIn I, const uint4* __restrict__ taps, int col_first,
                  unsigned col_tiles, unsigned per_ch, long long n_out, double scale, double g_start, double g_step,
                  int apply, float* __restrict__ out, size_t out_stride,
@@ -250,93 +310,88 @@ decim_mma_kernel(const MmaPlan M, const MmaIn I, const uint4* __restrict__ taps,
           (uint8_t)decision<kDop>(I, c, total - keep + k - I.tail_len);
     return;
   }
-  const int KS = M.B >> 4;                       // 16-decision steps of a block
-  const int pitch = 4 * KS + 4;                  // words of a column (its lanes on distinct banks)
+  const int ksh = 31 - __clz(M.B >> 4);          // 16-decision steps of a block: 2^ksh
+  const int KS = 1 << ksh;
   const long long n0 = col_first + (long long)bx * kMmaCols;
   const int cols = kMmaCols + 16 * M.T;          // columns n0 - 16 T .. n0 + 127
-  for (int k = tid; k < cols * KS; k += blockDim.x) {
-    const int col = k / KS, ks = k % KS;
-    const long long i = (n0 - 16 * M.T + col) * M.B + 16 * ks;
-    unsigned w = 0u;
-    uint4 sel;
-    if (i >= 0 && i + 16 <= I.count) {
-      if (kDop) {
-        w = dop_word(I.dop[(size_t)c * I.stride + (i >> 4)]);
-      } else {
-        const uint8_t* b = I.bits + (size_t)c * I.stride + i;
+  // selectors as [step][column][4 lanes]: a fragment is 32 consecutive words,
+  // and the columns of the next product lie at a fixed distance; a step's rows
+  // are 16 bytes further than whole, so that the words of one column (written
+  // by neighbouring threads) fall on different banks
+  const int pitch = 4 * cols + 4;
+  const long long i0 = (n0 - 16 * M.T) * M.B;
+  constexpr int kLoads = 4;                      // words of a thread on their way at once
+  for (int k0 = tid; k0 < cols * KS; k0 += kLoads * 32 * kMmaWarps) {
+    unsigned w[kLoads], none[kLoads];
 #pragma unroll
-        for (int u = 0; u < 16; u++) w |= (unsigned)(b[u] & 1u) << (15 - u);
-      }
-      sel = make_uint4(sel4(w, 0), sel4(w, 1), sel4(w, 2), sel4(w, 3));
-    } else {
-      unsigned none = 0u;
-      for (int u = 0; u < 16; u++) {
-        const unsigned d = decision<kDop>(I, c, i + u);
-        w |= (d & 1u) << (15 - u);
-        none |= (d >> 1) << (15 - u);
-      }
-      auto with = [&](int q) {
-        const unsigned t = none >> (6 - 2 * q);
-        const unsigned a = (t >> 9) & 1u, b = (t >> 8) & 1u, e = (t >> 1) & 1u, f = t & 1u;
-        const unsigned m = (a * 0x000000ffu) | (b * 0x0000ff00u) | (e * 0x00ff0000u) | (f * 0xff000000u);
-        return (sel4(w, q) & ~m) | (kSelNone & m);
-      };
-      sel = make_uint4(with(0), with(1), with(2), with(3));
+    for (int u = 0; u < kLoads; u++) {
+      const int k = k0 + u * 32 * kMmaWarps;
+      const long long i = i0 + 16ll * k;
+      w[u] = none[u] = 0u;
+      if (k >= cols * KS) continue;
+      if (kDop && i >= 0 && i + 16 <= I.count)
+        w[u] = __float_as_uint(I.dop[(size_t)c * I.stride + (i >> 4)]);
     }
-    *reinterpret_cast<uint4*>(&mma_smem[col * pitch + 4 * ks]) = sel;
+#pragma unroll
+    for (int u = 0; u < kLoads; u++) {
+      const int k = k0 + u * 32 * kMmaWarps;
+      const long long i = i0 + 16ll * k;
+      if (k >= cols * KS) continue;
+      unsigned wr = 0u;                          // bit b: decision b of the word
+      if (i >= 0 && i + 16 <= I.count) {
+        if (kDop) {
+          wr = __brev(dop_word(__uint_as_float(w[u]))) >> 16;
+        } else {
+          const uint8_t* b = I.bits + (size_t)c * I.stride + i;
+#pragma unroll
+          for (int e = 0; e < 16; e++) wr |= (unsigned)(b[e] & 1u) << e;
+        }
+      } else {
+        for (int e = 0; e < 16; e++) {
+          const unsigned d = decision<kDop>(I, c, i + e);
+          wr |= (d & 1u) << e;
+          none[u] |= (d >> 1) << e;
+        }
+      }
+      uint4 sel = make_uint4(sel4(wr, 0), sel4(wr, 1), sel4(wr, 2), sel4(wr, 3));
+      if (none[u]) {
+        auto blank = [&](unsigned v, int q) {    // bytes of the decisions that are not there
+          const unsigned m = ((none[u] << 4) >> (2 * q)), o = ((none[u] << 3) >> (2 * q));
+          const unsigned at = (__byte_perm(m, o, 0x5140) & 0x10101010u) >> 4;
+          return (v & ~(at * 0xffu)) | (kSelNone & (at * 0xffu));
+        };
+        sel = make_uint4(blank(sel.x, 0), blank(sel.y, 1), blank(sel.z, 2), blank(sel.w, 3));
+      }
+      *reinterpret_cast<uint4*>(&mma_smem[(k & (KS - 1)) * pitch + 4 * (k >> ksh)]) = sel;
+    }
   }
   __syncthreads();
-  // product tiles: one digit of one output phase a warp at a time
-  const int groups = kMmaDigits * M.F;
+  // product tiles: two digits of one output phase over a third of the columns
+  // a warp (the decisions' fragments cost as much as a product, so each serves
+  // two; the last pair has one digit)
+  const int dg = 2 * (warp / kMmaParts), part = warp % kMmaParts;
   const int steps = M.T * KS;
-  for (int g0 = 0; g0 < groups; g0 += kMmaWarps) {
-    const int g = g0 + warp;                     // (phase, digit)
-    float acc[kMmaAcc / 8][4];
-#pragma unroll
-    for (int n = 0; n < kMmaAcc / 8; n++)
-#pragma unroll
-      for (int r = 0; r < 4; r++) acc[n][r] = 0.0f;
-    const uint4* A = taps + ((size_t)g * steps) * 32 + lane;
-    uint4 an = A[0];
-    const unsigned* sb = mma_smem + (lane >> 2) * pitch + (lane & 3);
-    for (int st = 0; st < steps; st++) {
-      const uint4 a = an;
-      if (st + 1 < steps) an = A[(size_t)(st + 1) * 32];
-      const int t = st / KS, ks = st - t * KS;
-      const unsigned* col = sb + 16 * (M.T - 1 - t) * pitch + 4 * ks;
-#pragma unroll
-      for (int n = 0; n < kMmaAcc / 8; n++) {
-        const unsigned sel = col[8 * n * pitch];
-        const unsigned b0 = __byte_perm(kPool, 0u, sel), b1 = __byte_perm(kPool, 0u, sel >> 16);
-        asm volatile(
-            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
-            "{%8,%9}, {%0,%1,%2,%3};"
-            : "+f"(acc[n][0]), "+f"(acc[n][1]), "+f"(acc[n][2]), "+f"(acc[n][3])
-            : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
-      }
-    }
-    // the diagonals: y[n] = sum_i acc[i][n - i], whole numbers below 2^24.
-    // The tiles lie behind the selectors, which further phases still read.
-    float* tile = reinterpret_cast<float*>(mma_smem + cols * pitch) + warp * 16 * kAccRow;
-    int* sums = reinterpret_cast<int*>(mma_smem + cols * pitch) + kMmaWarps * 16 * kAccRow;
-#pragma unroll
-    for (int n = 0; n < kMmaAcc / 8; n++) {
-      float* p = tile + (lane >> 2) * kAccRow + 8 * n + 2 * (lane & 3);
-      *reinterpret_cast<float2*>(p) = make_float2(acc[n][0], acc[n][1]);
-      *reinterpret_cast<float2*>(p + 8 * kAccRow) = make_float2(acc[n][2], acc[n][3]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int n = 0; n < kMmaCols / 32; n++) {
+  // the tiles lie behind the selectors, which further phases still read
+  float* const tiles = reinterpret_cast<float*>(mma_smem + KS * pitch);
+  int* const sums = reinterpret_cast<int*>(tiles + kMmaDigits * 16 * kAccRow);
+  for (int ph = 0; ph < M.F; ph++) {
+    const uint4* A = taps + ((size_t)(ph * kMmaDigits + dg) * steps) * 32 + lane;
+    const unsigned* sb = mma_smem + 64 * (M.T - 1) + 32 * kN * part + lane;
+    float* tile = tiles + dg * 16 * kAccRow + (lane >> 2) * kAccRow + 8 * kN * part + 2 * (lane & 3);
+    if (dg + 1 < kMmaDigits) mma_tile<2>(A, steps, KS, pitch, sb, tile);
+    else mma_tile<1>(A, steps, KS, pitch, sb, tile);
+    __syncthreads();
+    for (int k = tid; k < kMmaDigits * kMmaCols; k += 32 * kMmaWarps) {
+      const int at = k % kMmaCols;
+      const float* tile = tiles + k / kMmaCols * 16 * kAccRow;
       float y = 0.0f;
 #pragma unroll
-      for (int i = 0; i < 16; i++) y += tile[i * kAccRow + 16 + 32 * n + lane - i];
-      sums[warp * kMmaCols + 32 * n + lane] = (int)y;
+      for (int i = 0; i < 16; i++) y += tile[i * kAccRow + 16 + at - i];
+      sums[k] = (int)y;
     }
     __syncthreads();
-    // groups of one round are the digits of one phase, in the warps' order
     if (tid < kMmaCols) {
-      const long long m = (n0 + tid) * M.F + g0 / kMmaWarps;
+      const long long m = (n0 + tid) * M.F + ph;
       if (m < n_out) {
         long long y = 0;
 #pragma unroll
@@ -346,13 +401,13 @@ decim_mma_kernel(const MmaPlan M, const MmaIn I, const uint4* __restrict__ taps,
         out[(size_t)c * out_stride + m] = (float)v;
       }
     }
-    __syncthreads();
+    if (ph + 1 < M.F) __syncthreads();
   }
 }
 
 __host__ size_t mma_smem_bytes(const MmaPlan& M) {
-  return sizeof(unsigned) * (size_t)(kMmaCols + 16 * M.T) * (4 * (M.B >> 4) + 4) +
-         sizeof(float) * (size_t)kMmaWarps * 16 * kAccRow + sizeof(int) * kMmaWarps * kMmaCols;
+  return sizeof(unsigned) * (size_t)(M.B >> 4) * (4 * (kMmaCols + 16 * M.T) + 4) +
+         sizeof(float) * (size_t)kMmaDigits * 16 * kAccRow + sizeof(int) * kMmaDigits * kMmaCols;
 }
 
 // The plan of `stages` stages and its taps in the order of the A fragments:
