@@ -197,6 +197,84 @@ struct PcWalk {
   }
 };
 
+// The same step with fewer operations, for the walks that allow it.
+//   * Every cell of the table in (-1, 1] (every filter of the NTF table trains
+//     such a one: its cells stay below 0.92) leaves the sign of y - c the sign
+//     of y, so the output is the sign of v and neither history nor table is
+//     read.
+//   * The products with the g that are zero in the table's filters (the even
+//     ones at odd orders, the odd ones at even orders) are left out, which
+//     changes nothing while the states are finite.
+//   * Components 0 .. 2, which a running modulator keeps far inside the
+//     limiter, are not clamped but watched: `peak` collects their magnitudes.
+//   * v's sign bit stands for v >= 0: with y = +-1 and a_0 > 0, x + a_0 d_0 is
+//     never -0 (t_0 - y and a cancelling sum are +0), and so neither is v; v is
+//     not NaN while the watched components stay below the limit.
+// A chunk that passed the limit or met a value that is not finite is run again
+// by step().  What bounds the walk is the instructions of its one warp, about
+// 1.8 cycles each (ncu; 72 of them in step()), and the chain of one output to
+// the next (the sum v behind d_0, 9 operations).  CLANS-7 with the limiter: 52.6
+// -> 38.3 ns a sample (two chains of v for both signs of y, picked by the last
+// output, or the sign by a comparison: 40.0 and above).
+template <int N>
+__host__ __device__ constexpr bool pc_g_zero(int i) { return (i & 1) == ((N & 1) ? 0 : 1); }
+constexpr int kPcWatched = 3;
+constexpr unsigned kPcPlainCodes = 5u;   // two codes of 1: output 1 for v >= 0, else 0
+
+__device__ __forceinline__ float pc_max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(fabsf(b)), "f"(fabsf(c)));
+  return r;
+}
+
+// y: the previous output (+-1), replaced by this step's
+template <int N, bool LIM>
+__device__ __forceinline__ void pc_plain_step(PcWalk<N, LIM>& W, float x, float& y, float& peak) {
+  float (&s)[10] = W.s;
+  float d[10];
+  float t0 = s[0];
+  if (!pc_g_zero<N>(0)) t0 = __fsub_rn(t0, __fmul_rn(W.C.g[0], s[1]));
+  t0 = __fadd_rn(t0, x);
+#pragma unroll
+  for (int i = 1; i < N - 1; i++) {
+    d[i] = __fadd_rn(s[i], s[i - 1]);
+    if (!pc_g_zero<N>(i)) d[i] = __fsub_rn(d[i], __fmul_rn(W.C.g[i], s[i + 1]));
+  }
+  d[N - 1] = __fadd_rn(s[N - 1], s[N - 2]);
+  d[0] = __fsub_rn(t0, y);
+  float v = __fadd_rn(x, __fmul_rn(W.C.a[0], d[0]));
+#pragma unroll
+  for (int i = 1; i < N; i++) v = __fadd_rn(v, __fmul_rn(W.C.a[i], d[i]));
+  y = __uint_as_float((__float_as_uint(v) & 0x80000000u) | 0x3f800000u);
+  constexpr int M = N < kPcWatched ? N : kPcWatched;
+  peak = pc_max3(peak, d[0], M > 1 ? d[1] : d[0]);
+  if (M > 2) peak = fmaxf(peak, fabsf(d[2]));
+  if (LIM) {
+#pragma unroll
+    for (int k = M; k < N; k++) d[k] = pc_clamp(d[k], -W.L, W.L);
+  }
+#pragma unroll
+  for (int k = 0; k < N; k++) s[k] = d[k];
+}
+
+// Whether a chunk of plain steps stands: the watched components inside the
+// limiter, every state finite (an infinite or NaN state stays one) and far from
+// overflow (16 sums from below 1e30 stay below 1e36).
+constexpr float kPcFar = 1.0e30f;
+constexpr int kPcHold = 24;   // chunks in step() after one that did not stand (a low limit: all of them)
+
+template <int N, bool LIM>
+__device__ __forceinline__ bool pc_stands(const PcWalk<N, LIM>& W, float peak) {
+  float z = 0.0f;
+  bool ok = peak <= (LIM ? fminf(W.L, kPcFar) : kPcFar);
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    z = __fadd_rn(z, __fmul_rn(W.s[k], 0.0f));
+    if (!LIM) ok = ok && fabsf(W.s[k]) <= kPcFar;
+  }
+  return ok && z == 0.0f;
+}
+
 // The first sample after a reset (prev_y = 0): the plain step.
 template <int N, bool LIM>
 __device__ __forceinline__ unsigned pc_first_step(PcWalk<N, LIM>& W, const uint8_t* row, float x) {
@@ -217,7 +295,7 @@ __device__ __forceinline__ unsigned pc_first_step(PcWalk<N, LIM>& W, const uint8
 }
 
 template <int N, bool LIM>
-__device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, PcState& st,
+__device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, bool plain, PcState& st,
                        const float* __restrict__ x, long long count, uint8_t* __restrict__ out) {
   PcWalk<N, LIM> W;
 #pragma unroll
@@ -236,6 +314,13 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, PcState& st,
     const unsigned pair = codes[ph0 * kPcHist + (int)(W.hist >> 1)];
     W.code = (W.hist & 1u) ? pair >> 2 : pair & 3u;
   }
+  // plain steps need the table's zero pattern of g, and finite states to start from
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    if (k <= N - 2 && pc_g_zero<N>(k) && W.C.g[k] != 0.0f) plain = false;
+    if (!(fabsf(W.s[k]) <= kPcFar)) plain = false;
+  }
+  if (!(W.C.a[0] > 1.0e-6f && W.C.a[0] < 1.0e3f)) plain = false;
   const bool any = count > 0;
   if (any && st.prev_y == 0.0f) {
     *out++ = (uint8_t)pc_first_step(W, codes + ((ph0 + 1) & 7) * kPcHist, *x++);
@@ -251,6 +336,7 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, PcState& st,
 #pragma unroll
   for (int j = 0; j < kPcAhead; j++) xa[j] = j < count ? x[j] : 0.0f;
   long long base = 0;
+  int hold = 0;   // chunks to go in whole steps after one that did not stand
   // whole chunks: straight-line code over kPcAhead samples, the next chunk's
   // inputs in flight meanwhile (converted when used)
   for (; base + kPcAhead <= count; base += kPcAhead) {
@@ -266,8 +352,37 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, PcState& st,
       }
     }
     unsigned w[kPcAhead / 4] = {0u, 0u, 0u, 0u};
+    bool stands = false;
+    if (plain && hold == 0) {
+      float keep[N];
 #pragma unroll
-    for (int j = 0; j < kPcAhead; j++) w[j >> 2] |= W.step(rows[j & 7], xa[j]) << (8 * (j & 3));
+      for (int k = 0; k < N; k++) keep[k] = W.s[k];
+      float peak = 0.0f, y = W.pbit ? 1.0f : -1.0f;
+      unsigned neg = 0u;   // the outputs' signs, the last in bit 0
+#pragma unroll
+      for (int j = 0; j < kPcAhead; j++) {
+        pc_plain_step<N, LIM>(W, xa[j], y, peak);
+        neg = __funnelshift_l(__float_as_uint(y), neg, 1);
+      }
+      stands = pc_stands<N, LIM>(W, peak);
+      if (stands) {
+        W.hist = ~neg & 0xffu;
+        W.pbit = ~neg & 1u;
+#pragma unroll
+        for (int k = 0; k < kPcAhead; k++)
+          w[k >> 2] |= ((~neg >> (kPcAhead - 1 - k)) & 1u) << (8 * (k & 3));
+      } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) W.s[k] = keep[k];
+        hold = kPcHold;
+      }
+    } else if (hold > 0) {
+      hold--;
+    }
+    if (!stands) {
+#pragma unroll
+      for (int j = 0; j < kPcAhead; j++) w[j >> 2] |= W.step(rows[j & 7], xa[j]) << (8 * (j & 3));
+    }
     if (vec_out) {
       *reinterpret_cast<uint4*>(out + base) = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
@@ -290,10 +405,10 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, PcState& st,
 }
 
 template <int N>
-__device__ __forceinline__ void pc_run_lim(const PcCoef& C, const uint8_t* codes, PcState& st,
+__device__ __forceinline__ void pc_run_lim(const PcCoef& C, const uint8_t* codes, bool plain, PcState& st,
                                            const float* x, long long count, uint8_t* out) {
-  if (C.limit > 0.0f) pc_run<N, true>(C, codes, st, x, count, out);
-  else pc_run<N, false>(C, codes, st, x, count, out);
+  if (C.limit > 0.0f) pc_run<N, true>(C, codes, plain, st, x, count, out);
+  else pc_run<N, false>(C, codes, plain, st, x, count, out);
 }
 
 __global__ void __launch_bounds__(32) precorr_process_kernel(const __grid_constant__ PcCoef C,
@@ -304,27 +419,29 @@ __global__ void __launch_bounds__(32) precorr_process_kernel(const __grid_consta
                                                              uint8_t* __restrict__ bits,
                                                              size_t bits_stride) {
   __shared__ uint8_t codes[kPcPhases * kPcHist];
+  bool plain = true;
   for (int i = threadIdx.x; i < kPcPhases * kPcHist; i += blockDim.x) {
     const int ph = i / kPcHist, h2 = (2 * (i % kPcHist)) & 0xFF;
     codes[i] = (uint8_t)(pc_code(table[h2 * kPcPhases + ph]) |
                          (pc_code(table[(h2 + 1) * kPcPhases + ph]) << 2));
+    plain = plain && codes[i] == kPcPlainCodes;
   }
-  __syncthreads();
+  plain = __syncthreads_and(plain);
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nch) return;
   PcState st = states[c];
   const float* x = in + (size_t)c * in_stride;
   uint8_t* o = bits + (size_t)c * bits_stride;
   switch (C.order) {
-    case 2: pc_run_lim<2>(C, codes, st, x, count, o); break;
-    case 3: pc_run_lim<3>(C, codes, st, x, count, o); break;
-    case 4: pc_run_lim<4>(C, codes, st, x, count, o); break;
-    case 5: pc_run_lim<5>(C, codes, st, x, count, o); break;
-    case 6: pc_run_lim<6>(C, codes, st, x, count, o); break;
-    case 7: pc_run_lim<7>(C, codes, st, x, count, o); break;
-    case 8: pc_run_lim<8>(C, codes, st, x, count, o); break;
-    case 9: pc_run_lim<9>(C, codes, st, x, count, o); break;
-    default: pc_run_lim<10>(C, codes, st, x, count, o); break;
+    case 2: pc_run_lim<2>(C, codes, plain, st, x, count, o); break;
+    case 3: pc_run_lim<3>(C, codes, plain, st, x, count, o); break;
+    case 4: pc_run_lim<4>(C, codes, plain, st, x, count, o); break;
+    case 5: pc_run_lim<5>(C, codes, plain, st, x, count, o); break;
+    case 6: pc_run_lim<6>(C, codes, plain, st, x, count, o); break;
+    case 7: pc_run_lim<7>(C, codes, plain, st, x, count, o); break;
+    case 8: pc_run_lim<8>(C, codes, plain, st, x, count, o); break;
+    case 9: pc_run_lim<9>(C, codes, plain, st, x, count, o); break;
+    default: pc_run_lim<10>(C, codes, plain, st, x, count, o); break;
   }
   states[c] = st;
 }
@@ -351,12 +468,14 @@ __global__ void __launch_bounds__(32) precorr_batch_kernel(const __grid_constant
                                                            const PcBatchRow* __restrict__ rows,
                                                            int nrows) {
   __shared__ uint8_t codes[kPcPhases * kPcHist];
+  bool plain = true;
   for (int i = threadIdx.x; i < kPcPhases * kPcHist; i += blockDim.x) {
     const int ph = i / kPcHist, h2 = (2 * (i % kPcHist)) & 0xFF;
     codes[i] = (uint8_t)(pc_code(table[h2 * kPcPhases + ph]) |
                          (pc_code(table[(h2 + 1) * kPcPhases + ph]) << 2));
+    plain = plain && codes[i] == kPcPlainCodes;
   }
-  __syncthreads();
+  plain = __syncthreads_and(plain);
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nrows) return;
   const PcBatchRow row = rows[r];
@@ -367,15 +486,15 @@ __global__ void __launch_bounds__(32) precorr_batch_kernel(const __grid_constant
   st.phase = 0;
   st.pad = 0;
   switch (C.order) {
-    case 2: pc_run_lim<2>(C, codes, st, row.in, row.count, row.out); break;
-    case 3: pc_run_lim<3>(C, codes, st, row.in, row.count, row.out); break;
-    case 4: pc_run_lim<4>(C, codes, st, row.in, row.count, row.out); break;
-    case 5: pc_run_lim<5>(C, codes, st, row.in, row.count, row.out); break;
-    case 6: pc_run_lim<6>(C, codes, st, row.in, row.count, row.out); break;
-    case 7: pc_run_lim<7>(C, codes, st, row.in, row.count, row.out); break;
-    case 8: pc_run_lim<8>(C, codes, st, row.in, row.count, row.out); break;
-    case 9: pc_run_lim<9>(C, codes, st, row.in, row.count, row.out); break;
-    default: pc_run_lim<10>(C, codes, st, row.in, row.count, row.out); break;
+    case 2: pc_run_lim<2>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 3: pc_run_lim<3>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 4: pc_run_lim<4>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 5: pc_run_lim<5>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 6: pc_run_lim<6>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 7: pc_run_lim<7>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 8: pc_run_lim<8>(C, codes, plain, st, row.in, row.count, row.out); break;
+    case 9: pc_run_lim<9>(C, codes, plain, st, row.in, row.count, row.out); break;
+    default: pc_run_lim<10>(C, codes, plain, st, row.in, row.count, row.out); break;
   }
 }
 

@@ -118,3 +118,34 @@ def test_precorr_orders(oracle, order):
     got = gpu.process_block(torch.from_numpy(x).cuda()).cpu().numpy()
     for c in range(2):
         assert np.array_equal(got[c], ref[c].process(x[c]))
+
+
+@pytest.mark.parametrize("name,limit", [("clans-7", 2.5), ("clans-7", 8.0), ("clans-6", 6.0),
+                                        ("clans-8", 0.0), ("sdm-5", 12.0)])
+def test_precorr_chunks_that_do_not_stand(oracle, name, limit):
+    """The walk's short step watches its first components instead of clamping
+    them: loud passages that reach the limiter, values that overflow, an
+    infinite and a NaN input, each between quiet stretches, in calls that cut
+    the 16-sample chunks."""
+    from foo_dsd_trellis_gb300 import ntf
+    from foo_dsd_trellis_gb300.precorr import PreCorr
+    f = ntf.get_filter(name, 5644800)
+    rng = np.random.default_rng(int(limit * 10) + f.order)
+    n = 6000
+    x = 0.4 * np.sin(2 * np.pi * 1e-3 * np.arange(n)) + 0.1 * rng.standard_normal(n)
+    x[1000:1200] *= 20.0
+    x[2000:2020] = 3e37 * rng.choice([-1.0, 1.0], 20)
+    x[3000:] = 0.0
+    x[3100] = -0.0
+    x[4000:] = 0.3 * rng.standard_normal(n - 4000)
+    x[5000] = np.inf
+    x[5500] = np.nan
+    x = x.astype(np.float32).astype(np.float64)
+    gpu = PreCorr(f.order, f.a, f.g, limit, num_channels=1)
+    ref = oracle.PreCorr(f.order, np.array(f.a), np.array(f.g), limit)
+    pos = 0
+    for ln in (7, 900, 1203, 17, 16, 2873, 984):
+        blk = x[pos:pos + ln]
+        pos += ln
+        got = gpu.process_block(torch.from_numpy(blk).cuda())[0].cpu().numpy()
+        np.testing.assert_array_equal(got, ref.process(blk), err_msg=str(pos))
