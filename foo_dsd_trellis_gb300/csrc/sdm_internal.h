@@ -25,6 +25,14 @@ __device__ __forceinline__ double clamp_state(double v, double lim) {
   return v;
 }
 
+// A coefficient for int_mul (sdm_intmul.h): its mantissa left-justified in 64
+// bits, and the exponent and sign words that a product takes over.
+struct IntCoef {
+  unsigned ch, cl;        // mantissa << 11
+  unsigned kc;            // (exponent - 1024) << 20
+  unsigned sign;          // sign bit
+};
+
 // Uniform trellis parameters (one NTF and one (K, depth, lat) per launch).
 struct SdmParams {
   double a[kMaxOrder];
@@ -41,6 +49,10 @@ struct SdmParams {
   // only by the failure-path tests, DSDGPU_OPT_FAILURE_TEST)
   int hop_limit;                // path-hash chain walk, hops
   long long part_wait_cycles;   // balanced launch: wait for an unpublished part
+  // the coefficients for products on the integer pipe (set by the launchers);
+  // int_ok 0: some coefficient or the limit is out of their range
+  IntCoef ia[kMaxOrder], ig[kMaxOrder];
+  int int_ok;
 };
 
 // Survivor selection strategy of the SDM kernel.

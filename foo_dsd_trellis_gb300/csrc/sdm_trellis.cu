@@ -26,6 +26,7 @@
 // reproduce the reference's slot memory, including the K = 32 store one past
 // act[] that lands on path_hash[0] while bank 1 is sorted (src/trellis.c:668-673).
 #include "sdm_internal.h"
+#include "sdm_intmul.h"
 
 #include <algorithm>
 #include <climits>
@@ -144,22 +145,24 @@ __device__ __forceinline__ int all_products(bool zg) {
 // Operation k of the shared part, inputs S[1..N-1] (a child's state), into
 // np (with scratch tg).  Orders respect the dependencies when k runs
 // 0, 1, 2, ...
-template <int N>
+template <int N, bool IM>
 __device__ __forceinline__ void shared_op(int k, const SdmParams& P, const double (&S)[N],
                                           Pack<N>& np, double (&tg)[N], bool zg) {
+  auto mulg = [&](int i, double x) { return IM ? int_mul(P.ig[i], x) : __dmul_rn(P.g[i], x); };
+  auto mula = [&](int i, double x) { return IM ? int_mul(P.ia[i], x) : __dmul_rn(P.a[i], x); };
   if (N < 3) {
-    if (k == 0) np.G0 = __dmul_rn(P.g[0], S[1]);
+    if (k == 0) np.G0 = mulg(0, S[1]);
     return;
   }
   constexpr int M = N - 3;   // middle indices i = 2..N-2
   constexpr int Z = mid_g<N>();
   if (k == 0) {
-    if (g_zero<N>(0)) np.G1 = __dmul_rn(P.g[1], S[2]);
-    else np.G0 = __dmul_rn(P.g[0], S[1]);
+    if (g_zero<N>(0)) np.G1 = mulg(1, S[2]);
+    else np.G0 = mulg(0, S[1]);
     return;
   }
   k -= 1;
-  if (k < Z) { const int i = mid_g_at<N>(k); tg[i] = __dmul_rn(P.g[i], S[i + 1]); return; }
+  if (k < Z) { const int i = mid_g_at<N>(k); tg[i] = mulg(i, S[i + 1]); return; }
   k -= Z;
   if (k < M) { const int i = 2 + k; np.D[i] = __dadd_rn(S[i], S[i - 1]); return; }
   k -= M;
@@ -178,7 +181,7 @@ __device__ __forceinline__ void shared_op(int k, const SdmParams& P, const doubl
         if (g_zero<N>(i)) np.D[i] = vsub(np.D[i], vmul(P.g[i], S[i + 1]));
     }
   }
-  if (k < N - 2) { const int i = 2 + k; np.A[i] = __dmul_rn(P.a[i], np.D[i]); return; }
+  if (k < N - 2) { const int i = 2 + k; np.A[i] = mula(i, np.D[i]); return; }
 }
 
 template <int N>
@@ -186,7 +189,7 @@ __device__ __forceinline__ void shared_all(const SdmParams& P, const double (&S)
                                            bool zg) {
   double tg[N];
 #pragma unroll
-  for (int k = 0; k < shared_ops<N>(); k++) shared_op<N>(k, P, S, np, tg, zg);
+  for (int k = 0; k < shared_ops<N>(); k++) shared_op<N, false>(k, P, S, np, tg, zg);
 }
 
 // Whether this filter's g has the zero pattern and no a is zero (a state that
@@ -376,7 +379,7 @@ __host__ __device__ constexpr int sort_stages() {
 // most of every FP64 warp instruction idle.  `lane` is the lane within the
 // job, `hm` the job's lanes; warp intrinsics use hm and width LPJ, ballots
 // are shifted to the job's bits.
-template <int N, int LPJ, int RW>
+template <int N, int LPJ, int RW, bool IM>
 __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restrict__ ctxs,
                         WarpSmem<LPJ>& sm, int* __restrict__ status) {
   constexpr int S = WarpSmem<LPJ>::S;
@@ -453,6 +456,9 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
   Pack<N> pk;
   pk.G0 = pk.G1 = 0.0;
   shared_all<N>(P, s, pk, zg);
+  // whether the states in hand are operands for integer products (a step that
+  // finds one that is not forms its products, and the next step's, in FP64)
+  bool int_in = false;
 
   // the traceback ring's word being written, and for the other words the lane
   // whose ring they were when that word was entered: they are moved between
@@ -611,7 +617,7 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     constexpr int kSortOps = (kOps < kStages ? kOps : kStages) > kDeferOps
                                  ? (kOps < kStages ? kOps : kStages) - kDeferOps : 0;
     word_sort<LPJ>(c0, c1, lane, hm, [&](int st) {
-      if (st < kSortOps) shared_op<N>(st, P, S, npk, tg, zg);
+      if (st < kSortOps) shared_op<N, IM>(st, P, S, npk, tg, zg);
     });
     int si0 = (int)(c0 & 63u), si1 = (int)(c1 & 63u);
     {
@@ -647,7 +653,27 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       }
     }
 #pragma unroll
-    for (int k = kSortOps; k < kOps; k++) shared_op<N>(k, P, S, npk, tg, zg);
+    for (int k = kSortOps; k < kOps; k++) shared_op<N, IM>(k, P, S, npk, tg, zg);
+    if (IM) {
+      // operands of this step's integer products and of the next one's (the
+      // clamped ones lie between them and the limit): out of range in some lane,
+      // or a filter out of range, and the shared part is formed in FP64
+      unsigned w = range_word(d1);
+#pragma unroll
+      for (int i = 2; i < N; i++) w = max(w, range_word(npk.D[i]));
+      bool in = !__any_sync(hm, live && w > kRangeSpan);
+      int z = in && int_in ? 0 : 1;
+      asm volatile("" : "+r"(z));
+#pragma unroll 1
+      for (; __builtin_expect(z > 0, 0); z--) {
+        shared_all<N>(P, S, npk, zg);
+        w = range_word(d1);
+#pragma unroll
+        for (int i = 2; i < N; i++) w = max(w, range_word(npk.D[i]));
+        in = !__any_sync(hm, live && w > kRangeSpan);
+      }
+      int_in = in && P.int_ok;
+    }
     const unsigned elig = want ? nx1 : (livemask & ~nx1);
     c_drop += 2ull * (unsigned)(n - __popc(elig));
     c_tot += 2ull * (unsigned)n;
@@ -994,7 +1020,7 @@ sdm_jobs_kernel(SdmParams P, const SdmJob* __restrict__ jobs, int njobs,
     j = __shfl_sync(hm, j, 0, LPJ);
     if (j >= njobs) break;
     const SdmJob job = jobs[j];
-    run_job<N, LPJ, kRegRingWords>(P, job, ctxs, sm, status);
+    run_job<N, LPJ, kRegRingWords, true>(P, job, ctxs, sm, status);
     __syncwarp(hm);
   }
 }
@@ -1015,7 +1041,7 @@ sdm_jobs_wide_kernel(SdmParams P, const SdmJob* __restrict__ jobs, int njobs,
     j = __shfl_sync(kFull, j, 0);
     if (j >= njobs) break;
     const SdmJob job = jobs[j];
-    run_job<N, 32, kRingWords>(P, job, ctxs, sm, status);
+    run_job<N, 32, kRingWords, false>(P, job, ctxs, sm, status);
     __syncwarp();
   }
 }
@@ -1106,7 +1132,7 @@ sdm_parts_kernel(SdmParams P, const SdmJob* __restrict__ jobs, long long part_le
       pj.seed_state = nullptr;
     }
     const bool more = off + pj.n_in < jb.n_in;
-    run_job<N, 32, kRegRingWords>(P, pj, ctxs, sm, status);
+    run_job<N, 32, kRegRingWords, true>(P, pj, ctxs, sm, status);
     __threadfence();   // this part's context and decisions before its successor's entry
     __syncwarp();
     if (lane == 0 && more) {
@@ -1115,6 +1141,19 @@ sdm_parts_kernel(SdmParams P, const SdmJob* __restrict__ jobs, long long part_le
     }
     __syncwarp();
   }
+}
+
+// The parameters with the coefficients' forms for products on the integer pipe.
+static SdmParams with_int(const SdmParams& P) {
+  SdmParams Q = P;
+  bool ok = P.state_limit == 0.0 || (P.state_limit > 1e-200 && P.state_limit < 1e200);
+  for (int i = 0; i < P.order; i++) {
+    const bool ga = int_coef(P.a[i], &Q.ia[i]), gg = int_coef(P.g[i], &Q.ig[i]);
+    ok = ok && ga;
+    if (i <= P.order - 2 && (i & 1) != ((P.order & 1) ? 0 : 1)) ok = ok && gg;
+  }
+  Q.int_ok = ok ? 1 : 0;
+  return Q;
 }
 
 __global__ void parts_queue_init_kernel(unsigned long long* queue, long long total, int njobs) {
@@ -1156,9 +1195,10 @@ long long sdm_parts_total(const SdmJob* jobs, int njobs, long long part_len) {
   return total;
 }
 
-int launch_sdm_parts(const SdmParams& P, const SdmJob* d_jobs, int njobs, long long part_len,
+int launch_sdm_parts(const SdmParams& P0, const SdmJob* d_jobs, int njobs, long long part_len,
                      unsigned long long* d_queue, long long total, int warps_per_pipe, int sms,
                      SdmCtx* d_ctxs, int* d_status, cudaStream_t stream) {
+  const SdmParams P = with_int(P0);
   parts_queue_init_kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(d_queue, total, njobs);
   note_kernel("sdm_parts_kernel", P.order);
   const dim3 grid((unsigned)(4 * warps_per_pipe * sms));
@@ -1285,9 +1325,10 @@ static int child_lanes(const SdmParams& P, int njobs) {
 // launches at K <= 16 take the child kernel by the rule above, and at K <= 2
 // with more jobs than that serves the per-thread kernel (sdm_scalar.cu, the
 // fewest FP64 instructions per job).
-int launch_sdm_jobs(const SdmParams& P, const SdmJob* d_jobs, int njobs, int* d_counter,
+int launch_sdm_jobs(const SdmParams& P0, const SdmJob* d_jobs, int njobs, int* d_counter,
                     SdmCtx* d_ctxs, int* d_status, int max_blocks, cudaStream_t stream) {
   if (njobs <= 0) return 0;
+  const SdmParams P = with_int(P0);
   if (P.lanes == 0 && max_blocks == 0) {
     const int cl = child_lanes(P, njobs);
     if (cl > 0) {
