@@ -229,6 +229,9 @@ struct WarpSmem {
   // a sample)
   static constexpr int kTab = 64 * LPJ;
   uint8_t tab[kTab];
+  // the run's counts (conv_fail, next_filter_drops, total_children), added to
+  // once a block: out of the step loop's registers
+  unsigned long long count[3];
 };
 
 // Lanes per job: the smallest power of two >= K (at least 2) is the tightest
@@ -424,13 +427,14 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     sm.key[b][j] = (long long)src->skey[b][j];
     sm.link[b][j] = src->slink[b][j];
   }
-  unsigned long long c_conv = 0, c_coll = 0, c_drop = 0, c_tot = 0;
-  if (job.copy_from < 0) {
-    c_conv = src->conv_fail;
-    c_coll = src->cands_collapse;
-    c_drop = src->next_filter_drops;
-    c_tot = src->total_children;
+  if (lane == 0) {
+    const bool go_on = job.copy_from < 0;
+    sm.count[0] = go_on ? src->conv_fail : 0ull;   // cands_collapse counts with it
+    sm.count[1] = go_on ? src->next_filter_drops : 0ull;
+    sm.count[2] = go_on ? src->total_children : 0ull;
   }
+  const unsigned long long coll_over =
+      job.copy_from < 0 ? src->cands_collapse - src->conv_fail : 0ull;
   __syncwarp(hm);
   if (job.seed_state) {
     // DAS temp seeding: every live candidate gets the estimated state, cost 0.
@@ -482,16 +486,19 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     if (lane < n_in) x_cur = in[lane];
     if (LPJ + lane < n_in) x_nxt = in[LPJ + lane];
   }
-  uint8_t obit = 0;
   int err = 0;
   const bool lim_on = P.state_limit > 0.0;
 
-  for (long long t = 0; t < n_in; t++) {
-    const int tl = (int)(t & (LPJ - 1));
-    if (tl == 0 && t > 0) {
-      x_cur = x_nxt;
-      x_nxt = (in && t + LPJ + lane < n_in) ? in[t + LPJ + lane] : 0.0;
-    }
+  for (long long t0 = 0; t0 < n_in; t0 += LPJ) {
+   // a block of LPJ inputs, one a lane (the next block's loads in flight)
+   const int tn = (int)(n_in - t0 < LPJ ? n_in - t0 : LPJ);
+   if (t0 > 0) {
+     x_cur = x_nxt;
+     x_nxt = (in && t0 + LPJ + lane < n_in) ? in[t0 + LPJ + lane] : 0.0;
+   }
+   unsigned obits = 0u, k_conv = 0u, k_drop = 0u, k_tot = 0u;
+#pragma unroll 1
+   for (int tl = 0; tl < tn; tl++) {
     const double x = __shfl_sync(hm, x_cur, tl, LPJ);
     const int nb = bank ^ 1;
     int next_pos = pos + 1;
@@ -592,8 +599,9 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     }
     const bool odd_key = live && ((unsigned)(key0 >> 32) >= 0x7ff00000u ||
                                   (unsigned)(key1 >> 32) >= 0x7ff00000u);
-    const bool bad = __any_sync(hm, odd_key);
-    if (bad) zg = false;   // the shared part below takes every product
+    // a state that is not finite shows in the cost; with integer products the
+    // shared part's range check finds it
+    if (!IM && __any_sync(hm, odd_key)) zg = false;
 
     // the children's shared part, spread over the sort's stages below
     Pack<N> npk;
@@ -624,20 +632,26 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       const unsigned after = __shfl_down_sync(hm, c0, 1, LPJ);
       const bool same = (c0 >> 6) == (c1 >> 6) && (c1 >> 6) != kWordNone;
       const bool same2 = lane < LPJ - 1 && (c1 >> 6) == (after >> 6) && (c1 >> 6) != kWordNone;
-      if (__any_sync(hm, same || same2) || bad) {
+      if (__any_sync(hm, same || same2 || odd_key)) {
         long long sk0 = live ? key0 : LLONG_MAX, sk1 = live ? key1 : LLONG_MAX;
         si0 = 2 * lane;
         si1 = 2 * lane + 1;
         full_sort<LPJ>(sk0, si0, sk1, si1, lane, hm);
       }
     }
+    // All candidates carry one traceback bit nearly always (they share their
+    // history lat samples back): it is the wanted one, every child is eligible,
+    // and without equal paths the sorted positions are the ranks.
+    const bool uni = (nx1 == 0u || nx1 == livemask) && !pany && P.mode == kModeFast;
+    int want = nx1 != 0u ? 1 : 0;
     const bool sl0 = (si0 >> 1) < n, sl1 = (si1 >> 1) < n;
+    if (!uni) {
     const int sn0 = (int)((nx1 >> (si0 >> 1)) & 1u);   // traceback bit of each sorted child
     const int sn1 = (int)((nx1 >> (si1 >> 1)) & 1u);
     const int votes1 = 2 * __popc(nx1);
     const int majority = (votes1 > 2 * n - votes1) ? 1 : 0;
     const int first = __shfl_sync(hm, si0, 0, LPJ);
-    int want = (int)((nx1 >> (first >> 1)) & 1u);
+    want = (int)((nx1 >> (first >> 1)) & 1u);
     if (want != majority) {
       __syncwarp(hm);
       const unsigned mA = BALLOT(sl0 && sn0 == majority);
@@ -651,6 +665,7 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
         const double cbm = __longlong_as_double(sm.key[nb][(at & 1) ? bB : bA]);
         if (cbm < __dmul_rn(__longlong_as_double(sm.key[nb][first]), 1.1)) want = majority;
       }
+    }
     }
 #pragma unroll
     for (int k = kSortOps; k < kOps; k++) shared_op<N, IM>(k, P, S, npk, tg, zg);
@@ -666,6 +681,10 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       asm volatile("" : "+r"(z));
 #pragma unroll 1
       for (; __builtin_expect(z > 0, 0); z--) {
+        bool nf = not_finite(d0) || not_finite(d1);
+#pragma unroll
+        for (int i = 2; i < N; i++) nf |= not_finite(pk.D[i]);
+        if (__any_sync(hm, live && nf)) zg = false;
         shared_all<N>(P, S, npk, zg);
         w = range_word(d1);
 #pragma unroll
@@ -675,8 +694,8 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       int_in = in && P.int_ok;
     }
     const unsigned elig = want ? nx1 : (livemask & ~nx1);
-    c_drop += 2ull * (unsigned)(n - __popc(elig));
-    c_tot += 2ull * (unsigned)n;
+    k_drop += 2u * (unsigned)(n - __popc(elig));
+    k_tot += 2u * (unsigned)n;
 
     // ---- 2b. fast selection ----
     // Without equal paths, the reference's ordered insertion with path-hash
@@ -709,22 +728,34 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
         rem1 = BALLOT(dup && key_less(o1, ps, key1, lane));
       }
     }
-    const bool f0 = sl0 && ((elig >> (si0 >> 1)) & 1u) &&
-                    !((((si0 & 1) ? rem1 : rem0) >> (si0 >> 1)) & 1u);
-    const bool f1 = sl1 && ((elig >> (si1 >> 1)) & 1u) &&
-                    !((((si1 & 1) ? rem1 : rem0) >> (si1 >> 1)) & 1u);
-    const unsigned EA = BALLOT(f0), EB = BALLOT(f1);
-    const int m2 = __popc(EA) + __popc(EB);
+    bool f0 = sl0, f1 = sl1;
+    unsigned EA = livemask, EB = livemask;
+    int m2 = 2 * n;
+    if (!uni) {
+      f0 = sl0 && ((elig >> (si0 >> 1)) & 1u) &&
+           !((((si0 & 1) ? rem1 : rem0) >> (si0 >> 1)) & 1u);
+      f1 = sl1 && ((elig >> (si1 >> 1)) & 1u) &&
+           !((((si1 & 1) ? rem1 : rem0) >> (si1 >> 1)) & 1u);
+      EA = BALLOT(f0);
+      EB = BALLOT(f1);
+      m2 = __popc(EA) + __popc(EB);
+    }
     int f_cnt = 0, f_Ls = -1, f_link0 = -1, f_link1 = -1;
     long long f_Lk = LLONG_MAX;
     bool f_h0 = false, f_h1 = false;
     if (links_matter && m2 > K && __any_sync(hm, me && (q & (kBuckets - 1)) == 0)) fast_ok = false;
     if (fast_ok) {
       const unsigned below = (1u << lane) - 1u;
-      const int r0 = __popc(EA & below) + __popc(EB & below);
-      const int r1 = r0 + (f0 ? 1 : 0);
-      if (f0 && r0 < K) sm.act[r0] = (int8_t)si0;
-      if (f1 && r1 < K) sm.act[r1] = (int8_t)si1;
+      int u0 = 0, u1 = 0;
+      if (uni) {
+        u0 = __shfl_sync(hm, si0, lane >> 1, LPJ);
+        u1 = __shfl_sync(hm, si1, lane >> 1, LPJ);
+      } else {
+        const int r0 = __popc(EA & below) + __popc(EB & below);
+        const int r1 = r0 + (f0 ? 1 : 0);
+        if (f0 && r0 < K) sm.act[r0] = (int8_t)si0;
+        if (f1 && r1 < K) sm.act[r1] = (int8_t)si1;
+      }
       if (links_matter) {
         // eligible children sorted before, with a lower index: OR-scan of
         // one-hot index masks over the sorted positions
@@ -745,7 +776,7 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       __syncwarp(hm);
       f_cnt = m2 < K ? m2 : K;
       if (lane < f_cnt) {
-        f_Ls = sm.act[lane];
+        f_Ls = uni ? ((lane & 1) ? u1 : u0) : (int)sm.act[lane];
         f_Lk = sm.key[nb][f_Ls];
       }
       if (links_matter) {
@@ -903,7 +934,7 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     cs0 = __dadd_rn(fd0, hh ? -1.0 : 1.0);
     if (lim_on) cs0 = clamp_state(cs0, P.state_limit);
     cs1 = fS1;
-    if (t == n_in - 1) {
+    if (t0 + tl == n_in - 1) {
       // the full child state is only needed when the context is stored
       if (surv) {
         dst->s[lane][0] = cs0;
@@ -944,20 +975,20 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       }
     }
     __syncwarp(hm);
-    if (n_new < n_old) { c_conv++; c_coll++; }
+    k_conv += n_new < n_old ? 1u : 0u;
     n = n_new;
     bank = nb;
     pos = next_pos;
-
-    // ---- output ----
-    if (t >= job.skip_out) {
-      const long long o = t - job.skip_out;
-      const int ol = (int)(o & (LPJ - 1));
-      if (lane == ol) obit = (uint8_t)want;
-      if (ol == LPJ - 1 || t == n_in - 1) {
-        if (lane <= ol) job.out[o - ol + lane] = obit;
-      }
-    }
+    obits |= (unsigned)want << tl;
+   }
+   // ---- output: the block's decisions, and its counts ----
+   const long long o = t0 + lane - job.skip_out;
+   if (lane < tn && o >= 0) job.out[o] = (uint8_t)((obits >> lane) & 1u);
+   if (lane == 0) {
+     sm.count[0] += k_conv;
+     sm.count[1] += k_drop;
+     sm.count[2] += k_tot;
+   }
   }
 
   // ---- store the context (the states were stored at the last sample) ----
@@ -993,17 +1024,19 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
     dst->n = n;
     dst->bank = bank;
     dst->pos = pos;
-    dst->conv_fail = c_conv;
-    dst->cands_collapse = c_coll;
-    dst->next_filter_drops = c_drop;
-    dst->total_children = c_tot;
+    dst->conv_fail = sm.count[0];
+    dst->cands_collapse = sm.count[0] + coll_over;
+    dst->next_filter_drops = sm.count[1];
+    dst->total_children = sm.count[2];
   }
   err = __reduce_max_sync(hm, err);
   if (err && lane == 0) atomicMax(status, err);
 }
 
-template <int N, int LPJ>
-__global__ void __launch_bounds__(32, LPJ == 32 ? 13 : 10)
+// kCtas: CTAs that an SM must hold (at 32 lanes 13, which leaves 128 registers
+// and some spills, or 12 and 168; a launch takes 12 where its CTAs fit).
+template <int N, int LPJ, int kCtas>
+__global__ void __launch_bounds__(32, kCtas)
 sdm_jobs_kernel(SdmParams P, const SdmJob* __restrict__ jobs, int njobs,
                 int* __restrict__ job_counter, SdmCtx* __restrict__ ctxs,
                 int* __restrict__ status, int groups) {
@@ -1095,7 +1128,7 @@ __device__ __noinline__ unsigned long long wait_entry(const unsigned long long* 
 }
 
 template <int N>
-__global__ void __launch_bounds__(32, 13)
+__global__ void __launch_bounds__(32, 12)
 sdm_parts_kernel(SdmParams P, const SdmJob* __restrict__ jobs, long long part_len,
                  unsigned long long* __restrict__ queue, long long total,
                  SdmCtx* __restrict__ ctxs, int* __restrict__ status) {
@@ -1236,7 +1269,7 @@ static int launch_wide(const SdmParams& P, dim3 grid, const SdmJob* d_jobs, int 
   return 0;
 }
 
-template <int LPJ>
+template <int LPJ, int kCtas>
 static int launch_lpj(const SdmParams& P, dim3 grid, const SdmJob* d_jobs, int njobs,
                       int* d_counter, SdmCtx* d_ctxs, int* d_status, int groups,
                       cudaStream_t stream) {
@@ -1244,7 +1277,7 @@ static int launch_lpj(const SdmParams& P, dim3 grid, const SdmJob* d_jobs, int n
   switch (P.order) {
 #define DSD_CASE(NN)                                                                       \
   case NN:                                                                                 \
-    sdm_jobs_kernel<NN, LPJ><<<grid, 32, smem, stream>>>(P, d_jobs, njobs, d_counter, d_ctxs, \
+    sdm_jobs_kernel<NN, LPJ, kCtas><<<grid, 32, smem, stream>>>(P, d_jobs, njobs, d_counter, d_ctxs, \
                                                          d_status, groups);                \
     break;
     DSD_CASE(2) DSD_CASE(3) DSD_CASE(4) DSD_CASE(5) DSD_CASE(6)
@@ -1358,11 +1391,17 @@ int launch_sdm_jobs(const SdmParams& P0, const SdmJob* d_jobs, int njobs, int* d
   }
   note_kernel("sdm_jobs_kernel", P.order, lanes);
   switch (lanes) {
-    case 32: rc = launch_lpj<32>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
-    case 16: rc = launch_lpj<16>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
-    case 8: rc = launch_lpj<8>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
-    case 4: rc = launch_lpj<4>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
-    default: rc = launch_lpj<2>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    case 32:
+      // one job alone 4,986 cycles a step against 5,366; a plan's classes share
+      // the SMs, 16 CTAs each (16 mixed streams: 928 ms with 12)
+      rc = max_blocks == 0 && blocks <= 12 * (resident_warps() / 16)
+               ? launch_lpj<32, 12>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream)
+               : launch_lpj<32, 13>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream);
+      break;
+    case 16: rc = launch_lpj<16, 10>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    case 8: rc = launch_lpj<8, 10>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    case 4: rc = launch_lpj<4, 10>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
+    default: rc = launch_lpj<2, 10>(P, grid, d_jobs, njobs, d_counter, d_ctxs, d_status, groups, stream); break;
   }
   if (rc) return rc;
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
