@@ -451,20 +451,40 @@ adj_full_lane_kernel(LoopCoef C, const double* __restrict__ u, const uint8_t* __
 // loop without quantiser feedback is slightly unstable (the delayed
 // resonators have |eigenvalue| > 1), so only the exact operation sequence of
 // the trellis reproduces its bounded states; a reordered evaluation would
-// amplify rounding.  Writes the checkpoints, beta_t = y^_t - kappa v^_t and
-// the largest |state| seen (a sanity bound the host checks).
+// amplify rounding.
+//
+// Only the states are serial, so the walk is two kernels: base_state_kernel
+// runs a clip from end to end with the decisions fixed and writes the
+// checkpoints (four FP64 instructions a sample); base_full_kernel runs every
+// block from its checkpoint at once and writes beta_t = y^_t - kappa v^_t and
+// the largest |state| seen (a sanity bound the host checks), the ten or so
+// that nothing waits for.  Bound: the state chain's FP64 instructions at 64
+// cycles each.  65,536 samples of 16 clips: 47 ms as one kernel, NN ms as two.
 //
 // The |state| maximum is taken on the integer pipe (magnitudes of doubles
 // order like their bit patterns; a NaN state reads as above every bound).
 //
-// One clip per group of G lanes, one state component per lane (the same
-// operations per component as the reference's loop; v's sum stays left to
-// right on the gathered products).
+// One clip (or block) per group of G lanes, one state component per lane (the
+// same operations per component as the reference's loop; v's sum stays left to
+// right on the gathered products; adding -0.0 leaves any value as it is).
+
+// FP64 operations that stay where they are written (an FP64 instruction holds
+// its unit for 64 cycles: the order decides what waits).
+__device__ __forceinline__ double vadd(double a, double b) {
+  double r;
+  asm volatile("add.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+__device__ __forceinline__ double vmul(double a, double b) {
+  double r;
+  asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  return r;
+}
+
 template <int N, int G>
-__global__ void base_lane_kernel(LoopCoef C, const double* __restrict__ u,
-                                 const uint8_t* __restrict__ bits, long long n, int Lb, int nclips,
-                                 double* __restrict__ starts, double* __restrict__ beta,
-                                 double* __restrict__ smax) {
+__global__ void base_state_kernel(LoopCoef C, const double* __restrict__ u,
+                                  const uint8_t* __restrict__ bits, long long n, int Lb, int nclips,
+                                  double* __restrict__ starts) {
   Lane<G> L;
   long long item;
   lane_setup<G>(L, item);
@@ -472,22 +492,61 @@ __global__ void base_lane_kernel(LoopCoef C, const double* __restrict__ u,
   const int c = (int)item, k = L.k;
   const bool own = k < N;
   const double gk = own ? C.g[k] : 0.0;
-  const double ak = own ? C.a[k] : 0.0;
-  const size_t base = (size_t)c * n;
   const int nb = (int)(n / Lb);
-  const double* uc = u + base;
-  const uint8_t* bc = bits + base;
-  double s = 0.0;
+  const double* uc = u + (size_t)c * n;
+  const uint8_t* bc = bits + (size_t)c * n;
+  // G inputs and decisions, one a lane, the next ones on their way
+  double xl = k < n ? __ldg(uc + k) : 0.0;
+  int bl = k < n ? (int)__ldg(bc + k) : 0;
+  double s = 0.0, np = -0.0;   // np: -g_k s_{k+1} of the sample to come
+  for (long long t0 = 0; t0 < n; t0 += G) {
+    if ((t0 & (Lb - 1)) == 0 && own) starts[((size_t)c * nb + (size_t)(t0 / Lb)) * N + k] = s;
+    const long long tn = t0 + G + k;
+    const double xn = tn < n ? __ldg(uc + tn) : 0.0;
+    const int bn = tn < n ? (int)__ldg(bc + tn) : 0;
+    const int m = (int)min((long long)G, n - t0);
+#pragma unroll 2
+    for (int j = 0; j < m; j++) {
+      const double x = __shfl_sync(L.hm, xl, j, G);
+      const int y = __shfl_sync(L.hm, bl, j, G);
+      const double sp = __shfl_up_sync(L.hm, s, 1, G);
+      const double last = k == 0 ? x : (k < N - 1 ? np : -0.0);
+      const double ny = k == 0 ? (y ? -1.0 : 1.0) : -0.0;
+      const double uu = vadd(s, k == 0 ? np : (own ? sp : 0.0));
+      const double d = vadd(uu, last);
+      s = vadd(d, ny);
+      np = -vmul(gk, __shfl_down_sync(L.hm, d, 1, G));   // s_{k+1} = d_{k+1} for every k
+    }
+    xl = xn;
+    bl = bn;
+  }
+}
+
+template <int N, int G>
+__global__ void base_full_kernel(LoopCoef C, const double* __restrict__ u,
+                                 const uint8_t* __restrict__ bits, long long n, int Lb, int nclips,
+                                 const double* __restrict__ starts, double* __restrict__ beta,
+                                 unsigned long long* __restrict__ smax) {
+  Lane<G> L;
+  long long item;
+  lane_setup<G>(L, item);
+  const int nb = (int)(n / Lb);
+  if (item >= (long long)nclips * nb) return;          // whole groups leave together
+  const int c = (int)(item / nb), b = (int)(item % nb), k = L.k;
+  const bool own = k < N;
+  const double gk = own ? C.g[k] : 0.0;
+  const double ak = own ? C.a[k] : 0.0;
+  const size_t base = (size_t)c * n + (size_t)b * Lb;
+  double s = own ? starts[(size_t)item * N + k] : 0.0;
   unsigned long long mx = 0;
-  for (long long t = 0; t < n; t++) {
-    if ((t & (Lb - 1)) == 0 && own) starts[((size_t)c * nb + (size_t)(t / Lb)) * N + k] = s;
-    const double x = __ldg(uc + t);
+  for (int t = 0; t < Lb; t++) {
+    const double x = __ldg(u + base + t);
     const double d = loop_d_lane<N, G>(C, L, gk, s, x);
     const double p = __dmul_rn(ak, d);
     double v = __dadd_rn(x, __shfl_sync(L.hm, p, 0, G));
 #pragma unroll
     for (int j = 1; j < N; j++) v = __dadd_rn(v, __shfl_sync(L.hm, p, j, G));
-    const double yt = __ldg(bc + t) ? 1.0 : -1.0;
+    const double yt = __ldg(bits + base + t) ? 1.0 : -1.0;
     if (k == 0) beta[base + t] = yt - C.kappa * v;
     s = k == 0 ? __dsub_rn(d, yt) : d;
     if (own) {
@@ -500,7 +559,7 @@ __global__ void base_lane_kernel(LoopCoef C, const double* __restrict__ u,
     const unsigned long long other = __shfl_down_sync(L.hm, mx, o, G);
     mx = other > mx ? other : mx;
   }
-  if (k == 0) smax[c] = __longlong_as_double((long long)mx);
+  if (k == 0) atomicMax(smax + c, mx);
 }
 
 // ---- loss: decimating low-pass of (y - r), block partial sums of z^2 ----
@@ -747,11 +806,15 @@ int launch_scan(const char* which, dsdgpu_diff* D, const LoopCoef& C, const Mat&
   cudaStream_t s = D->c->stream;
   const int Lb = D->p.checkpoint;
   if (!strcmp(which, "base")) {
-    // one clip per warp, one state component per lane
+    // one state component per lane: one clip per warp, then all blocks
     constexpr int GB = N <= 8 ? 8 : 16;
-    base_lane_kernel<N, GB><<<D->p.nclips, GB, 0, s>>>(C, u, D->d_bits, D->n, Lb, D->p.nclips,
-                                                       D->d_starts, D->d_beta, D->d_smax);
-    D->c->launches -= 2;
+    cudaMemsetAsync(D->d_smax, 0, sizeof(double) * (size_t)D->p.nclips, s);
+    base_state_kernel<N, GB><<<D->p.nclips, GB, 0, s>>>(C, u, D->d_bits, D->n, Lb, D->p.nclips,
+                                                        D->d_starts);
+    base_full_kernel<N, GB><<<grid_of((long long)tot * GB, 32), 32, 0, s>>>(
+        C, u, D->d_bits, D->n, Lb, D->p.nclips, D->d_starts, D->d_beta,
+        (unsigned long long*)D->d_smax);
+    D->c->launches -= 1;
   } else if (!strcmp(which, "sur")) {
     sur_local_kernel<N><<<g, kScanThreads, 0, s>>>(C, u, beta, D->n, Lb, D->nb, D->p.nclips, D->d_ends);
     fwd_carry_kernel<N><<<gc, 32, 0, s>>>(carry, D->d_ends, D->nb, D->p.nclips, D->d_sstarts);
