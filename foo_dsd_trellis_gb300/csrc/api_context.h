@@ -122,7 +122,8 @@ struct dsdgpu_context {
   std::string sdm_last_kernel;              // ... and its kernel
 
   int* d_counter = nullptr;   // persistent-kernel job counter
-  int* d_status = nullptr;    // device status word (bounded walks/waits)
+  int* h_status = nullptr;   // the device status word, in mapped host memory
+  int* d_status = nullptr;   // its device address
 
   // trellis SDM
   bool sdm_ready = false;

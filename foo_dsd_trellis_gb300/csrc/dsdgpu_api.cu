@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 
 namespace dsdgpu {
@@ -100,11 +101,11 @@ int dsdgpu_context::ensure_scratch(size_t bytes) {
 int dsdgpu_context::check_status() {
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "stream synchronize");
-  int st = 0;
-  e = cudaMemcpy(&st, d_status, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "status read");
+  // the word lies in mapped host memory: the kernels' writes are visible once
+  // the stream is drained, without a copy (10 us a call)
+  const int st = *(volatile int*)h_status;
   if (st != 0) {
-    cudaMemset(d_status, 0, sizeof(int));
+    *(volatile int*)h_status = 0;
     char buf[128];
     snprintf(buf, sizeof buf, "device status word %d (bounded walk/wait gave up)", st);
     last_error = buf;
@@ -194,6 +195,63 @@ void dsdgpu_context::plan_steps(int64_t pend, int64_t count, int64_t discard, in
   sdm_plan_steps(sdm.lat, pend, count, discard, skip, out, new_pend);
 }
 
+namespace {
+
+// The contexts' status words in mapped host memory, a cache line each: up to 64
+// share one page (pinning memory takes 0.25 ms, more than the rest of a
+// context), which goes back with the last of them; further contexts pin their
+// own.
+class StatusWords {
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!page_) {
+      if (cudaHostAlloc(&page_, kWords * kLine, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        page_ = nullptr;
+        return nullptr;
+      }
+      used_ = 0;
+    }
+    for (int i = 0; i < kWords; i++)
+      if (!((used_ >> i) & 1ull)) {
+        used_ |= 1ull << i;
+        int* w = (int*)(page_ + i * kLine);
+        *w = 0;
+        return w;
+      }
+    int* w = nullptr;
+    if (cudaHostAlloc(&w, kLine, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    *w = 0;
+    return w;
+  }
+  void give(int* w) {
+    std::lock_guard<std::mutex> lock(mu_);
+    const ptrdiff_t at = (char*)w - page_;
+    if (!page_ || at < 0 || at >= kWords * kLine) {
+      cudaFreeHost(w);
+      return;
+    }
+    used_ &= ~(1ull << (at / kLine));
+    if (used_ == 0) {
+      cudaFreeHost(page_);
+      page_ = nullptr;
+    }
+  }
+
+ private:
+  static constexpr int kWords = 64, kLine = 64;
+  std::mutex mu_;
+  char* page_ = nullptr;
+  unsigned long long used_ = 0;
+};
+
+StatusWords& status_words() {
+  static StatusWords* w = new StatusWords;   // outlives contexts destroyed at exit
+  return *w;
+}
+
+}  // namespace
+
 extern "C" {
 
 int dsdgpu_create(int device, dsdgpu_context_t** out) {
@@ -208,8 +266,8 @@ int dsdgpu_create(int device, dsdgpu_context_t** out) {
   c->device = device;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMalloc(&c->d_counter, sizeof(int)) != cudaSuccess ||
-      cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess) {
+      (c->h_status = status_words().take()) == nullptr ||
+      cudaHostGetDevicePointer((void**)&c->d_status, c->h_status, 0) != cudaSuccess) {
     dsdgpu_destroy(c);
     return DSDGPU_ERR_CUDA;
   }
@@ -227,7 +285,7 @@ void dsdgpu_destroy(dsdgpu_context_t* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   c->release_all();
   if (c->d_counter) cudaFree(c->d_counter);
-  if (c->d_status) cudaFree(c->d_status);
+  if (c->h_status) status_words().give(c->h_status);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

@@ -197,3 +197,28 @@ def test_close_twice_and_destroy_null():
     g.close()
     g.close()
     _lib.load().dsdgpu_destroy(None)
+
+
+def test_many_contexts_keep_their_own_status():
+    """More contexts than share a page of status words, destroyed out of order:
+    each reports its own failure (a chain walk cut short by the failure option)
+    and nobody else's."""
+    from foo_dsd_trellis_gb300 import _lib, ntf
+    from foo_dsd_trellis_gb300.sdm import TrellisSdm
+    f = ntf.get_filter("clans-7", 6144000)
+    sdms = [TrellisSdm(f.order, f.a, f.g, 64, 32, 64, num_contexts=1) for _ in range(70)]
+    x = torch.from_numpy(multitone(4000, 41) * 2.0).cuda()
+    for bad in (0, 63, 64, 69):
+        sdms[bad].set_option(_lib.OPT_FAILURE_TEST, _lib.FAIL_CHAIN_WALK)
+        sdms[bad].set_select(_lib.SELECT_EXACT)
+        with pytest.raises(_lib.DsdGpuError):
+            sdms[bad].process_block(x)
+        sdms[bad].set_option(_lib.OPT_FAILURE_TEST, 0)
+        sdms[bad].reset()
+        sdms[bad].process_block(x)
+        sdms[(bad + 1) % 70].process_block(x)
+    for i in list(range(0, 70, 2)) + list(range(69, 0, -2)):
+        sdms[i].close()
+    again = TrellisSdm(f.order, f.a, f.g, 64, 32, 64, num_contexts=1)
+    again.process_block(x)
+    again.close()
