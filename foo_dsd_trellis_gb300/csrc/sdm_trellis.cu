@@ -1317,13 +1317,14 @@ static int child_ops(int N, int H) {
 
 // Lanes of the child kernel (sdm_child.h) for a launch of njobs jobs without a
 // block cap, or 0 for the other kernels.  With w warps a scheduler a step takes
-// about 66 cycles an FP64 instruction and 800 more (w <= 1), or 76 w cycles an
-// FP64 instruction (the FP64 unit is the SM's: 19 cycles a warp instruction)
-// and 650 more; fewer lanes a job are more instructions a step over fewer
-// warps.  Measured cycles a step at order 6, by lanes a job:
+// about 66 cycles an FP64 instruction and 640 to 1,080 more (by lanes a child),
+// or 76 w cycles an FP64 instruction (the FP64 unit is the SM's: 19 cycles a
+// warp instruction) and 650 more; fewer lanes a job are more instructions a
+// step over fewer warps.  Measured cycles a step at order 6, by lanes a job:
 //   K = 2:  430 jobs 1,630 / 1,873 / 2,379 / 2,748 at 32 / 16 / 8 / 4 lanes,
-//           1,722 jobs 4,241 / 2,571 / 2,628 / 3,011
-//   K = 4:  608 jobs 1,887 / 2,565 / 2,935 at 32 / 16 / 8, 1,216 jobs 3,162 / 2,790 / 3,040
+//           1,722 jobs 4,241 / 2,542 / 2,710 / 3,011, 2,000 jobs - / 2,921 / 2,819
+//   K = 4:  608 jobs 1,879 / 2,607 / 2,935 at 32 / 16 / 8, 861 jobs 2,403 / 2,676,
+//           1,216 jobs 3,154 / 2,791 / 3,040
 //   K = 8:  608 jobs 2,504 / 3,215 at 32 / 16, 1,216 jobs 4,414 / 3,393
 // The warp kernel's step (one candidate a lane, its selection in sequence with
 // its arithmetic) takes 5,500 cycles alone and 8,925 at order 8 with 2.47 warps
@@ -1337,8 +1338,10 @@ static int child_lanes(const SdmParams& P, int njobs) {
   int best = 0;
   double cost = 1e300;
   for (int lanes = 32; lanes >= 2 * KC; lanes >>= 1) {
-    const double ops = child_ops(N, lanes / (2 * KC)), w = warps(32 / lanes);
-    const double c = std::max(66.0 * ops + 800.0, 76.0 * ops * w + 650.0);
+    const int H = lanes / (2 * KC);
+    const double ops = child_ops(N, H), w = warps(32 / lanes);
+    const double alone = H >= 8 ? 640.0 : H == 4 ? 760.0 : H == 2 ? 1080.0 : 1000.0;
+    const double c = std::max(66.0 * ops + alone, 76.0 * ops * w + 650.0);
     if (c < cost) { cost = c; best = lanes; }
   }
   double other = 1e300;
