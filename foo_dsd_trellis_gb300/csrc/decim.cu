@@ -746,7 +746,12 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
     delete s;
     return c->cuda_fail(cudaGetLastError(), "decimation buffers");
   }
-  const int smem = (int)mma_smem_bytes(s->mma);
+  // The attribute belongs to the kernel, not to the context: the widest plan's
+  // size, so that no context's setup takes another's away.
+  MmaPlan widest = s->mma;
+  widest.B = 1 << kMaxStages;
+  widest.T = 4;   // 62 blocks of lags, and no plan has more
+  const int smem = (int)mma_smem_bytes(widest);
   if (cudaFuncSetAttribute(decim_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
       cudaFuncSetAttribute(decim_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
     delete s;

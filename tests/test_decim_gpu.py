@@ -162,3 +162,31 @@ def test_decim_dop_equals_bits(oracle):
         assert n == m.value
         assert torch.equal(a, b), frames
     L.dsdgpu_destroy(h)
+
+
+def test_decim_contexts_of_different_ratios(oracle):
+    """A context's setup leaves the contexts that were set up before it usable:
+    ratios from 512 down to 2, then all run, the widest first."""
+    from foo_dsd_trellis_gb300 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(12)
+    ratios = (512, 128, 16, 2)
+    hs = []
+    for D in ratios:
+        h = C.c_void_p()
+        assert L.dsdgpu_create(0, C.byref(h)) == 0
+        _lib.check(h, L.dsdgpu_decim_setup(h, 44100 * D, 44100, 1))
+        hs.append(h)
+    for D, h in zip(ratios, hs):
+        n = 40 * max(D, 16)
+        bits = (rng.random(n) > 0.4).astype(np.uint8)
+        d = torch.from_numpy(bits).cuda()
+        out = torch.zeros(n // D, dtype=torch.float32, device="cuda")
+        m = C.c_size_t()
+        _lib.check(h, L.dsdgpu_decim_process(h, 1, C.c_void_p(d.data_ptr()), n, n,
+                                             C.c_void_p(out.data_ptr()), n // D, 1.0, 1.0, C.byref(m)))
+        want = oracle.Decimator(44100 * D, 44100).process(bits.astype(np.float64) * 2 - 1)
+        assert m.value == len(want)
+        np.testing.assert_allclose(out.cpu().numpy(), want, rtol=0, atol=2e-7, err_msg=str(D))
+    for h in hs:
+        L.dsdgpu_destroy(h)
