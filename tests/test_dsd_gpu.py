@@ -223,3 +223,32 @@ def test_dsd_rate_conversion_das_glue(oracle, fs_in, fs_out):
                                 seg_len=32768, seed_mode=0, reposition=True)
     assert np.array_equal(out[:, :ns].cpu().numpy(), want)
     enc.close()
+
+
+@pytest.mark.parametrize("taps", [1, 2, 64, 255, 256])
+def test_boxcar_tile_edges(oracle, taps):
+    """The boxcar's tiles (1,792 outputs, 8 inputs a thread): calls that end
+    before, on and behind their edges, rows at every alignment, gain constant
+    and ramped, the history across calls longer and shorter than the window."""
+    import ctypes as C
+    from foo_dsd_trellis_gb300 import _lib
+    L = _lib.load()
+    h = C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    nch = 3
+    _lib.check(h, L.dsdgpu_boxcar_setup(h, taps, nch))
+    refs = [oracle.Boxcar(taps) for _ in range(nch)]
+    rng = np.random.default_rng(taps)
+    for k, n in enumerate((1, 7, 1791, 1792, 1793, 255, 3585, 2048, 5000)):
+        g0, g1 = ((0.708, 0.708), (1.0, 1.0), (0.25, 0.9))[k % 3]
+        bits = (rng.random((nch, n + k)) > 0.4).astype(np.uint8)
+        d = torch.from_numpy(bits).cuda()
+        out = torch.full((nch, n + 3), 7.0, dtype=torch.float64, device="cuda")
+        _lib.check(h, L.dsdgpu_boxcar_process(h, 0, nch, C.c_void_p(d.data_ptr()), d.stride(0), n,
+                                              C.c_void_p(out.data_ptr()), out.stride(0), g0, g1))
+        got = out.cpu().numpy()
+        for c in range(nch):
+            want = refs[c].process(bits[c, :n].astype(np.float32) * 2 - 1, g0, g1)
+            np.testing.assert_array_equal(got[c, :n], want, err_msg=f"{n} {c}")
+            assert (got[c, n:] == 7.0).all()
+    L.dsdgpu_destroy(h)
