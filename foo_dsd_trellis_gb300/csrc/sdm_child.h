@@ -37,8 +37,16 @@
 // kernel at K <= 4, the warp kernel above): K = 2, order 6 2,668 -> 1,498;
 // K = 4 4,720 -> 1,659; K = 8, depth 4 5,548 -> 2,500; K = 16, order 8
 // 5,630 -> 2,883.
+//
+// With one lane a child (H = 1) the step has the most FP64 instructions, and
+// with several warps a scheduler the FP64 unit's rate is all there is: there the
+// products go to the integer pipe (sdm_intmul.h), a third of the FP64
+// instructions.  Measured cycles a step, products in FP64 -> on the integer pipe:
+// K = 16, order 8 2,883 -> 2,790 with one job, 7,600 -> 5,697 with 1,500; K = 2,
+// order 6 3,011 -> 2,186 with 1,722 jobs; K = 8 3,393 -> 2,567 with 1,216.
 #pragma once
 #include "sdm_internal.h"
+#include "sdm_intmul.h"
 
 #include <climits>
 
@@ -67,14 +75,14 @@ __device__ __forceinline__ double neg(double v) {
 }
 
 // FP64 operations of the advance
-template <int N, int H, int C>
+template <int N, int H, int C, bool IM>
 __host__ __device__ constexpr int advance_ops() {
   int m = 0, d = 1;
   for (int j = 0; j < C; j++) {
     m += need_g<N, H, C>(j) ? 1 : 0;
     d += need_g<N, H, C>(j) && j > 0 ? 1 : 0;
   }
-  return m + (H == 1 && !need_g<N, H, C>(0) ? C - 1 : C) + d + C + N;
+  return (IM ? 0 : m + C) + (H == 1 && !need_g<N, H, C>(0) ? C - 1 : C) + d + N;
 }
 
 // FP64 operations that stay where they are written: an FP64 instruction holds
@@ -177,8 +185,10 @@ __host__ __device__ inline size_t ring_words(int lat, int KC) {
 // the advance of this lane's candidate or child by input x: d and v.  The
 // operations that do not wait for one another come first; hook(k) runs behind
 // the k-th.
-template <int N, int H, int C, typename Hook>
-__device__ __forceinline__ void advance(const double (&st)[C], double x, double (&d)[C], double& v,
+// IM (H = 1): the products on the integer pipe, those with a one at a time in
+// the shadow of v's sums.
+template <int N, int H, int C, bool IM, typename Hook>
+__device__ __forceinline__ void advance(const SdmParams& P, const double (&st)[C], double x, double (&d)[C], double& v,
                                         const double (&gl)[C], const double (&al)[C], double d0, int q,
                                         int lane0, bool zg, Hook&& hook) {
   constexpr bool kPad = H * C > N;
@@ -193,8 +203,13 @@ __device__ __forceinline__ void advance(const double (&st)[C], double x, double 
   for (int j = 0; j < C; j++) {
     mm[j] = 0.0;
     if (need_g<N, H, C>(j)) {
-      mm[j] = neg(vmul(gl[j], j < C - 1 ? st[j + 1 < C ? j + 1 : j] : sn_q));
-      hook(k++);
+      const double sn = j < C - 1 ? st[j + 1 < C ? j + 1 : j] : sn_q;
+      if (IM) {
+        mm[j] = neg(int_mul(P.ig[j], sn));
+      } else {
+        mm[j] = neg(vmul(gl[j], sn));
+        hook(k++);
+      }
     }
   }
 #pragma unroll
@@ -242,25 +257,35 @@ __device__ __forceinline__ void advance(const double (&st)[C], double x, double 
     for (int j = 0; j < C; j++)
       if (q * C + j >= N) d[j] = 0.0;
   }
-#pragma unroll
-  for (int j = 0; j < C; j++) {
-    p[j] = vmul(al[j], d[j]);
-    hook(k++);
-  }
   double acc = x;
-  double pn = H == 1 ? p[0] : __shfl_sync(kFull, p[0], lane0);
+  if constexpr (IM) {
+    p[0] = int_mul(P.ia[0], d[0]);
 #pragma unroll
-  for (int i = 0; i < N; i++) {
-    const double pi = pn;
-    const int i1 = i + 1 < N ? i + 1 : i;
-    if (i + 1 < N) pn = H == 1 ? p[i1 % C] : __shfl_sync(kFull, p[i1 % C], lane0 + i1 / C);
-    acc = vadd(acc, pi);
-    hook(k++);
+    for (int j = 0; j < N; j++) {
+      acc = vadd(acc, p[j]);
+      if (j + 1 < N) p[j + 1] = int_mul(P.ia[j + 1], d[j + 1]);
+      hook(k++);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < C; j++) {
+      p[j] = vmul(al[j], d[j]);
+      hook(k++);
+    }
+    double pn = H == 1 ? p[0] : __shfl_sync(kFull, p[0], lane0);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const double pi = pn;
+      const int i1 = i + 1 < N ? i + 1 : i;
+      if (i + 1 < N) pn = H == 1 ? p[i1 % C] : __shfl_sync(kFull, p[i1 % C], lane0 + i1 / C);
+      acc = vadd(acc, pi);
+      hook(k++);
+    }
   }
   v = acc;
 }
 
-template <int N, int KC, int H>
+template <int N, int KC, int H, bool IM>
 __global__ void __launch_bounds__(32, 12)
 sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__ jobs, int njobs,
                  SdmCtx* __restrict__ ctxs, int* __restrict__ status) {
@@ -357,6 +382,7 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
   }
   int perm = r;   // the candidate this one descends from when the ring's word was entered
 
+  bool int_in = false;   // IM: the states in hand are operands for integer products
   bool zg;        // the structurally zero products may be left out
   {
     bool ok = true;
@@ -372,7 +398,7 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
     zg = __all_sync(kFull, ok);
   }
 
-  constexpr int kOps = advance_ops<N, H, C>();
+  constexpr int kOps = advance_ops<N, H, C, IM>();
 
   const long long n_in = job.n_in;
   long long n_max = n_in;
@@ -418,7 +444,7 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
     }
   }
   __syncwarp();
-  if (n_max > 0) advance<N, H, C>(s, s_x[js][0], d, v, gl, al, s[0], q, lane0, zg, [](int) {});
+  if (n_max > 0) advance<N, H, C, false>(P, s, s_x[js][0], d, v, gl, al, s[0], q, lane0, zg, [](int) {});
 
   // steps from step t to the next at which a job leaves its ring's word or ends
   auto next_event = [&](long long t) {
@@ -653,11 +679,30 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
     };
     constexpr int kPieces = kP + 3;
     double dn[C], vn;
-    advance<N, H, C>(s, x1, dn, vn, gl, al, first, q, lane0, zg, [&](int k) {
+    advance<N, H, C, IM>(P, s, x1, dn, vn, gl, al, first, q, lane0, zg, [&](int k) {
       if (k < kPieces) piece(k);
     });
 #pragma unroll
     for (int k = kOps; k < kPieces; k++) piece(k);
+    if (IM) {
+      // operands of the integer products (the clamped ones lie between them and
+      // the limit): out of range in some lane, and the advance is formed in FP64
+      auto in_range = [&]() {
+        unsigned w = range_word(dn[0]);
+#pragma unroll
+        for (int j = 1; j < C; j++) w = max(w, range_word(dn[j]));
+        return !__any_sync(kFull, live && w > kRangeSpan);
+      };
+      bool in = in_range();
+      int z = in && int_in ? 0 : 1;
+      asm volatile("" : "+r"(z));
+#pragma unroll 1
+      for (; DSD_RARE(z > 0); z--) {
+        advance<N, H, C, false>(P, s, x1, dn, vn, gl, al, first, q, lane0, zg, [](int) {});
+        in = in_range();
+      }
+      int_in = in;
+    }
 
     // ---- commit: the survivors' advance ----
     const int sl = jb + ac * H;
@@ -756,17 +801,22 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
   if (err && wl == 0) atomicMax(status, err);
 }
 
-template <int KC, int H>
+template <int KC, int H, bool IM = false>
 int launch(const SdmParams& P, const SdmJob* d_jobs, int njobs, SdmCtx* d_ctxs, int* d_status,
            cudaStream_t stream) {
+  // one lane has all of a child's components: its step is bound by its FP64
+  // instructions, and the products go to the integer pipe
+  if constexpr (H == 1 && !IM) {
+    if (P.int_ok) return launch<KC, H, true>(P, d_jobs, njobs, d_ctxs, d_status, stream);
+  }
   const int jpw = 32 / (2 * KC * H);
   const dim3 grid((unsigned)((njobs + jpw - 1) / jpw)), block(32);
   const size_t smem = sizeof(uint32_t) * ring_words(P.lat, KC) * (size_t)jpw;
   switch (P.order) {
 #define DSD_CASE(NN)                                                                          \
   case NN:                                                                                    \
-    sdm_child_kernel<NN, KC, H><<<grid, block, smem, stream>>>(P, d_jobs, njobs, d_ctxs,      \
-                                                               d_status);                     \
+    sdm_child_kernel<NN, KC, H, IM><<<grid, block, smem, stream>>>(P, d_jobs, njobs, d_ctxs,  \
+                                                                   d_status);                 \
     break;
     DSD_CASE(2) DSD_CASE(3) DSD_CASE(4) DSD_CASE(5) DSD_CASE(6)
     DSD_CASE(7) DSD_CASE(8) DSD_CASE(9) DSD_CASE(10)

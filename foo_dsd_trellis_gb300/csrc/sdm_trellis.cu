@@ -1300,7 +1300,7 @@ int launch_sdm_child_large(const SdmParams& P, int lanes, const SdmJob* d_jobs, 
 // component of a lane the product with g (where a lane has one that is not
 // structurally zero), the two sums and the product with a; v; and e, its
 // square, the cost, s_0 and the cost's normalisation.
-static int child_ops(int N, int H) {
+static int child_ops(int N, int H, bool im) {
   const int C = (N + H - 1) / H;
   int m = 0, d = 1;
   for (int j = 0; j < C; j++) {
@@ -1312,23 +1312,25 @@ static int child_ops(int N, int H) {
     m += need;
     d += need && j > 0;
   }
-  return m + C + d + C + N + 5;
+  return (im ? 0 : m + C) + C + d + N + 5;
 }
 
 // Lanes of the child kernel (sdm_child.h) for a launch of njobs jobs without a
 // block cap, or 0 for the other kernels.  With w warps a scheduler a step takes
-// about 66 cycles an FP64 instruction and 640 to 1,080 more (by lanes a child),
+// about 66 cycles an FP64 instruction and 640 to 1,300 more (by lanes a child
+// and, at one, whether its products are formed on the integer pipe),
 // or 76 w cycles an FP64 instruction (the FP64 unit is the SM's: 19 cycles a
 // warp instruction) and 650 more; fewer lanes a job are more instructions a
 // step over fewer warps.  Measured cycles a step at order 6, by lanes a job:
-//   K = 2:  430 jobs 1,630 / 1,873 / 2,379 / 2,748 at 32 / 16 / 8 / 4 lanes,
-//           1,722 jobs 4,241 / 2,542 / 2,710 / 3,011, 2,000 jobs - / 2,921 / 2,819
-//   K = 4:  608 jobs 1,879 / 2,607 / 2,935 at 32 / 16 / 8, 861 jobs 2,403 / 2,676,
-//           1,216 jobs 3,154 / 2,791 / 3,040
-//   K = 8:  608 jobs 2,504 / 3,215 at 32 / 16, 1,216 jobs 4,414 / 3,393
+//   K = 2:  430 jobs 1,630 / 1,873 / 2,379 at 32 / 16 / 8 lanes,
+//           1,722 jobs 4,241 / 2,300 / 2,463 / 2,186 at 32 / 16 / 8 / 4,
+//           2,432 jobs 2,530 / 2,193 at 8 / 4, 4,864 jobs 2,252 at 4
+//   K = 4:  608 jobs 1,879 / 2,607 at 32 / 16, 1,216 jobs 3,154 / 2,675 / 2,570
+//           at 32 / 16 / 8, 4,000 jobs 3,189 at 8
+//   K = 8:  1 job 2,396 / 2,507 at 32 / 16, 608 jobs 2,504 / 2,525, 1,216 jobs 4,414 / 2,567
 // The warp kernel's step (one candidate a lane, its selection in sequence with
 // its arithmetic) takes 5,500 cycles alone and 8,925 at order 8 with 2.47 warps
-// a scheduler (the child kernel 7,600); the per-thread kernel (K <= 2) 9,600.
+// a scheduler (the child kernel 5,700); the per-thread kernel (K <= 2) 9,600.
 static int child_lanes(const SdmParams& P, int njobs) {
   const int K = P.cands, N = P.order;
   if (K > 16) return 0;
@@ -1339,8 +1341,10 @@ static int child_lanes(const SdmParams& P, int njobs) {
   double cost = 1e300;
   for (int lanes = 32; lanes >= 2 * KC; lanes >>= 1) {
     const int H = lanes / (2 * KC);
-    const double ops = child_ops(N, H), w = warps(32 / lanes);
-    const double alone = H >= 8 ? 640.0 : H == 4 ? 760.0 : H == 2 ? 1080.0 : 1000.0;
+    const bool im = H == 1 && P.int_ok;
+    const double ops = child_ops(N, H, im), w = warps(32 / lanes);
+    const double alone = H >= 8 ? 640.0 : H == 4 ? 760.0 : H == 2 ? 1080.0
+                         : !im ? 1000.0 : KC == 2 ? 820.0 : 1300.0;
     const double c = std::max(66.0 * ops + alone, 76.0 * ops * w + 650.0);
     if (c < cost) { cost = c; best = lanes; }
   }

@@ -499,3 +499,32 @@ def test_uneven_segments_share_warps(oracle, K, depth, lat, njobs, order):
         assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
             (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"]), i
         np.testing.assert_array_equal(q["best_state"], ctx.best_state())
+
+
+@pytest.mark.parametrize("K,order,njobs", [(2, 6, 3000), (1, 5, 5000), (4, 5, 2000), (8, 7, 1300),
+                                           (16, 8, 3), (9, 4, 700), (16, 6, 1300)])
+def test_products_in_and_out_of_range(oracle, K, order, njobs):
+    """At these numbers of jobs one lane has a child's whole state and forms its
+    products on the integer pipe, except while a state of the warp is not in
+    their range: fresh contexts (zero states) between running ones, silence,
+    levels of 1e-290 and 1e120, and all back in range."""
+    f = _ntf({4: "clans-4", 5: "sdm-5", 6: "clans-6", 7: "clans-7", 8: "clans-8"}[order],
+             2822400 if order == 4 else 5644800)
+    g = _gpu_sdm(f, 4, K, 40, nctx=njobs)
+    tail = 0.4 * multitone(150, seed=K)
+    rows = np.stack([np.concatenate([r, tail]) for r in (
+        np.zeros(100), np.full(100, 1e-290), 0.6 * multitone(100, seed=K), np.full(100, 1e120))])
+    refs = [_ora(oracle, f, 4, K, 40) for _ in range(8)]
+    for k, n in enumerate((50, 250)):   # first: every second group of four
+        lo = 0 if k else njobs // 2 // 4 * 4
+        idx = np.arange(lo, njobs)
+        xs = rows[idx % 4, :n]
+        got = g.process_block(torch.from_numpy(xs).cuda(), first=lo)
+        half = njobs // 2 // 4 * 4
+        for c in range(8):
+            fresh, row = c < 4, c % 4
+            if fresh and k == 0:
+                continue
+            want = oracle.sdm_bits(refs[c], rows[row, :n])
+            for i in np.flatnonzero(((idx < half) == fresh) & (idx % 4 == row))[::29]:
+                np.testing.assert_array_equal(got[i].cpu().numpy(), want, err_msg=f"{c} {n} {i}")
