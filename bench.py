@@ -57,6 +57,8 @@ WL = dict(workload="dsd128_das_stereo_10s_multitone_pink", fs_in=48000, fs_out=6
           l2="GPU arm: 512 MiB written between timed steps, outside the events; the CPU arm "
              "has no device cache to flush")
 FP64_OPS_PER_CAND_SAMPLE = 5 * WL["ntf_order"] + 6   # (2N+1) mul + (3N+5) add
+MEASURED_BF16_TFLOPS = 1926.4                         # MEASURED_PEAKS.json bf16_tflops
+FP64_ISSUED_PER_CAND_SAMPLE = 27                      # of them on the FP64 unit at N = 7
 SDM_DRAM_BYTES_PER_SAMPLE = 9.04                      # measured, see the traffic note below
 SDM_PARTS_DRAM_BYTES_PER_SAMPLE = 9.15                # the balanced launch's (parts kernel), measured
 
@@ -478,7 +480,10 @@ def run_ours(args):
     flops_per_sample = WL["cands"] * FP64_OPS_PER_CAND_SAMPLE
     flops = out_samples_step * flops_per_sample
     achieved = flops / sdm_s / 1e12
-    issued = sdm_samples * flops_per_sample / sdm_s / 1e12
+    # what the kernel puts on the FP64 unit: 27 warp instructions a step at
+    # N = 7 (the zero g products are left out, and the products of the part that
+    # both children share run on the integer pipe), so achieved can pass the peak
+    issued = sdm_samples * WL["cands"] * FP64_ISSUED_PER_CAND_SAMPLE / sdm_s / 1e12
     peak = fp64_peak / 1000.0
     sms = torch.cuda.get_device_properties(local).multi_processor_count
     sm_mhz = clk.get("sm_mhz") or 0.0
@@ -499,6 +504,7 @@ def run_ours(args):
                                        "sampled during the timed steps",
                 "sdm_input_samples_per_launch": sdm_samples,
                 "das_redundancy": sdm_samples / out_samples_step - 1.0,
+                "issued_ops_per_sample": WL["cands"] * FP64_ISSUED_PER_CAND_SAMPLE,
                 "issued_tflops": issued,
                 "issue_frac": issued / peak}
     # DRAM bytes per launch: ncu's dram__bytes per SDM input sample of the
@@ -1447,7 +1453,7 @@ def run_next(args):
         roof = {"bound": "fp64", "achieved": flops / sdm_s / 1e12, "peak": fp64_peak / 1000.0,
                 "unit": "TFLOP/s", "frac": flops / sdm_s / 1e12 / (fp64_peak / 1000.0),
                 "traffic": None,
-                "kernel": enc.last_sdm_kernel() + " (latency-bound small trellis)",
+                "kernel": enc.last_sdm_kernel(),
                 "algorithmic_flops_per_launch": flops, "flops_per_sample": cfg["cands"] * (5 * f.order + 6)}
     elif wl == "precorr128":
         pc_s = statistics.mean(sdm_ms) / 1000.0
@@ -1461,16 +1467,15 @@ def run_next(args):
                         "MEASURED_PEAKS hbm_gbs) is reported only for scale"}
     else:
         step_s = total_s / args.steps
-        # FP64 instructions: stage 1 = 4 table sums + the centre tap per output,
-        # stages 2-7 = 33 FMAs per output (the half-band's nonzero taps)
-        outs = [frames * 16 // 2 ** (k + 1) for k in range(cfg["stages"])]
-        instr = (5 * outs[0] + 33 * sum(outs[1:])) * nch
-        roof = {"bound": "fp64", "achieved": instr / step_s / 1e12, "peak": fp64_peak / 1000.0,
-                "unit": "T FP64 instructions/s", "frac": instr / step_s / 1e12 / (fp64_peak / 1000.0),
-                "traffic": None, "kernel": "decim_bits_kernel + decim_stage_kernel (7 stages, whole step timed)",
-                "algorithmic_instructions_per_launch": instr,
-                "per_output": "stage 1: 4 table reads + 5 DADD; stages 2-7: 33 DFMA (an FMA "
-                              "issues as one FP64 instruction; the probe's peak counts DADD/DMUL)"}
+        # the whole chain as one product: 7 digits of 8 bits x 64 lags a decision
+        flops = 2.0 * 448 * frames * 16 * nch
+        peak = MEASURED_BF16_TFLOPS
+        roof = {"bound": "tensor", "achieved": flops / step_s / 1e12, "peak": peak,
+                "unit": "TFLOP/s", "frac": flops / step_s / 1e12 / peak,
+                "traffic": None, "kernel": "decim_mma_kernel (whole step timed)",
+                "peak_source": "cuBLAS bf16 burst of MEASURED_PEAKS.json",
+                "algorithmic_flops_per_launch": flops,
+                "per_input": "448 multiply-adds a decision: seven 8-bit digits of the taps x 64 lags"}
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:
         cpu = _next_cpu(wl, inp, None, 0.5 if wl.startswith("samerate") else 1.0)
