@@ -259,7 +259,8 @@ __device__ __forceinline__ void advance(const SdmParams& P, const double (&st)[C
   }
   double acc = x;
   if constexpr (IM) {
-    p[0] = int_mul(P.ia[0], d[0]);
+    // without g_0 (odd orders) d_0 is 0 on every second step of a silence from rest
+    p[0] = need_g<N, H, C>(0) ? int_mul(P.ia[0], d[0]) : int_mul0(P.ia[0], d[0]);
 #pragma unroll
     for (int j = 0; j < N; j++) {
       acc = vadd(acc, p[j]);
@@ -688,7 +689,7 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
       // operands of the integer products (the clamped ones lie between them and
       // the limit): out of range in some lane, and the advance is formed in FP64
       auto in_range = [&]() {
-        unsigned w = range_word(dn[0]);
+        unsigned w = need_g<N, H, C>(0) ? range_word(dn[0]) : range_word0(dn[0]);
 #pragma unroll
         for (int j = 1; j < C; j++) w = max(w, range_word(dn[j]));
         return !__any_sync(kFull, live && w > kRangeSpan);

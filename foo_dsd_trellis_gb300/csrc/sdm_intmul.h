@@ -51,6 +51,17 @@ __device__ __forceinline__ double int_mul(const IntCoef& c, double s) {
   return __hiloint2double((int)(hi | ((sh ^ c.sign) & 0x80000000u)), (int)o0);
 }
 
+// The same with zeros in the operand's range.
+__device__ __forceinline__ bool is_zero(double s) {
+  return (2u * (unsigned)__double2hiint(s) | (unsigned)__double2loint(s)) == 0u;
+}
+__device__ __forceinline__ unsigned range_word0(double s) { return is_zero(s) ? 0u : range_word(s); }
+__device__ __forceinline__ double int_mul0(const IntCoef& c, double s) {
+  const double r = int_mul(c, s);
+  const double z = __hiloint2double((int)(((unsigned)__double2hiint(s) ^ c.sign) & 0x80000000u), 0);
+  return is_zero(s) ? z : r;
+}
+
 // Whether v may be a coefficient of int_mul, and its form.
 inline bool int_coef(double v, IntCoef* c) {
   unsigned long long b;
