@@ -616,10 +616,19 @@ int to_lines(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
 
 }  // namespace
 
+// Whether [a, a + na) and [b, b + nb) share a byte.
+static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+  return x < y + nb && y < x + na;
+}
+
 // One call of the decimation from DoP frames (d_dop, rows of `stride` floats)
 // or decision bytes (d_bits): the route by what the stream continues from (see
 // the head of the file).  DoP frames that have to take the stages are unpacked
-// into the context's scratch memory by the caller's `unpack` buffer.
+// into the context's scratch memory.  So is an input of the product that shares
+// memory with the output (a call in place): its CTAs read what others write
+// over.  (The stages have read the whole input before the first output is
+// written.)
 int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d_bits, size_t stride,
               size_t count, float* d_pcm, size_t pcm_stride, double gain_start, double gain_end,
               size_t* out_count) {
@@ -642,13 +651,38 @@ int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d
   const double step = n > 1 ? (gain_end - gs) / (double)(n - 1) : 0.0;
 
   const MmaPlan& M = s->mma;
+  const bool stages = s->from == dsdgpu_decim_state::kLines || s->ragged;   // at the start of the call
+  const bool all = stages && count < (size_t)128 * M.B;                     // and to its end
+  const size_t in_row = d_dop ? count / 16 * sizeof(float) : count;
+  const size_t in_step = d_dop ? stride * sizeof(float) : stride;
+  if (!all && n > 0 &&
+      overlap(d_dop ? (const void*)d_dop : d_bits, in_step * (size_t)(nch - 1) + in_row, d_pcm,
+              sizeof(float) * (pcm_stride * (size_t)(nch - 1) + n))) {
+    const size_t row = (count + 255) & ~(size_t)255;
+    int rc = c->ensure_scratch(row * (size_t)nch);
+    if (rc) return rc;
+    uint8_t* copy = (uint8_t*)c->d_scratch;
+    if (d_dop) {
+      rc = dsdgpu_dop_unpack(c, nch, d_dop, stride, count / 16, copy, row);
+      if (rc) return rc;
+    } else {
+      for (int ch = 0; ch < nch; ch++) {
+        const cudaError_t e = cudaMemcpyAsync(copy + row * (size_t)ch, d_bits + stride * (size_t)ch, count,
+                                              cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) return c->cuda_fail(e, "decimation input copy");
+      }
+    }
+    d_dop = nullptr;
+    d_bits = copy;
+    stride = row;
+  }
+
   int col_first = 0;
-  if (s->from == dsdgpu_decim_state::kLines || s->ragged) {
+  if (stages) {
     int rc = to_lines(c, s);
     if (rc) return rc;
     s->ragged = false;
     s->tail_len = 0;
-    const bool all = count < (size_t)128 * M.B;
     const size_t part = all ? count : (size_t)64 * M.B;
     const uint8_t* bits = d_bits;
     size_t bstride = stride;

@@ -190,3 +190,43 @@ def test_decim_contexts_of_different_ratios(oracle):
         np.testing.assert_allclose(out.cpu().numpy(), want, rtol=0, atol=2e-7, err_msg=str(D))
     for h in hs:
         L.dsdgpu_destroy(h)
+
+
+@pytest.mark.parametrize("fs_in,fs_out,nch", [(2822400, 176400, 2), (5644800, 44100, 3), (2822400, 1411200, 1)])
+def test_decim_in_place(oracle, fs_in, fs_out, nch):
+    """An output that lies in the input's memory (DoP frames replaced by their
+    PCM, decision bytes by theirs) is the same as in memory of its own: from
+    fresh state, after whole blocks and after a ragged end."""
+    from foo_dsd_trellis_gb300 import _lib, ntf
+    from foo_dsd_trellis_gb300.pipeline import Encoder
+    D = fs_in // fs_out
+    rng = np.random.default_rng(D + nch)
+    f = ntf.get_filter("clans-7", 5644800)
+    mk = lambda: Encoder(fs_in, fs_out, nch, f, 64, 32, 128, output_format=_lib.OUT_PCM)
+    L = _lib.load()
+    hs = [C.c_void_p(), C.c_void_p()]
+    for h in hs:
+        assert L.dsdgpu_create(0, C.byref(h)) == 0
+        _lib.check(h, L.dsdgpu_decim_setup(h, fs_in, fs_out, nch))
+    encs = [mk(), mk()] if D >= 16 else []
+    for frames in (65536, 8 * 4000 + 3, 8 * 3000):
+        n = 16 * frames // D
+        bits = (rng.random((nch, 16 * frames)) > 0.4).astype(np.uint8)
+        if encs:   # PCM no longer than its DoP frames
+            dop = torch.from_numpy(np.stack([oracle.dop_float_frames(bits[c], 0) for c in range(nch)])).cuda()
+            want = torch.zeros((nch, n), dtype=torch.float32, device="cuda")
+            encs[0].process(dop, want, 0.7, 0.9)
+            encs[1].process(dop, dop, 0.7, 0.9)
+            assert torch.equal(dop[:, :n], want), frames
+        raw = torch.zeros((nch, 64 * frames), dtype=torch.uint8, device="cuda")
+        raw[:, : 16 * frames] = torch.from_numpy(bits).cuda()
+        want = torch.zeros((nch, n), dtype=torch.float32, device="cuda")
+        m = C.c_size_t()
+        torch.cuda.synchronize()
+        for h, out, ostride in ((hs[0], want, n), (hs[1], raw, 16 * frames)):
+            _lib.check(h, L.dsdgpu_decim_process(h, nch, raw.data_ptr(), 64 * frames, 16 * frames,
+                                                 out.data_ptr(), ostride, 1.0, 1.0, C.byref(m)))
+            assert m.value == n
+        assert torch.equal(raw.view(torch.float32)[:, :n], want), frames
+    for h in hs:
+        L.dsdgpu_destroy(h)
