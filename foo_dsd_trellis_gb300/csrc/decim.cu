@@ -77,10 +77,12 @@ struct DecNz {
 constexpr int kLutGroups = 4;   // 32 even taps in groups of 8
 
 // FP64 stage: the 33 nonzero taps as FMAs in ascending tap order
+// (done: nothing is left to do where it is set, see to_lines)
 __global__ void decim_stage_kernel(const __grid_constant__ DecNz T, const double* __restrict__ in,
                                    size_t in_stride, long long m_out,
                                    const double* __restrict__ dly, double* __restrict__ out,
-                                   size_t out_stride, int nch) {
+                                   size_t out_stride, int nch, const int* __restrict__ done) {
+  if (done && *done) return;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m_out * nch) return;
   const long long c = i / m_out, m = i % m_out;
@@ -103,8 +105,10 @@ __global__ void __launch_bounds__(256) decim_bits_kernel(const __grid_constant__
                                                          size_t in_stride, long long m_out,
                                                          const double* __restrict__ dly,
                                                          double* __restrict__ out,
-                                                         size_t out_stride, int nch) {
+                                                         size_t out_stride, int nch,
+                                                         const int* __restrict__ done) {
   __shared__ double tab[kLutGroups * 256];
+  if (done && *done) return;
   for (int q = threadIdx.x; q < kLutGroups * 256; q += blockDim.x) tab[q] = lut[q];
   __syncthreads();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -139,9 +143,9 @@ __global__ void __launch_bounds__(256) decim_bits_kernel(const __grid_constant__
 template <bool kBits>
 __global__ void decim_dly_kernel(const uint8_t* __restrict__ bits, const double* __restrict__ in,
                                  size_t in_stride, long long used, double* __restrict__ dly,
-                                 int nch) {
+                                 int nch, const int* __restrict__ done) {
   const int c = blockIdx.x;
-  if (c >= nch) return;
+  if (c >= nch || (done && *done)) return;
   __shared__ double tmp[kDecTaps - 1];
   double* dl = dly + (size_t)c * (kDecTaps - 1);
   for (int k = threadIdx.x; k < kDecTaps - 1; k += blockDim.x) {
@@ -154,6 +158,13 @@ __global__ void decim_dly_kernel(const uint8_t* __restrict__ bits, const double*
   __syncthreads();
   for (int k = threadIdx.x; k < kDecTaps - 1; k += blockDim.x) dl[k] = tmp[k];
 }
+
+// the delay lines at rest, unless `done`; and `done` itself
+__global__ void decim_rest_kernel(double* __restrict__ dly, int n, const int* __restrict__ done) {
+  if (*done) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dly[i] = 0.0;
+}
+__global__ void decim_done_kernel(int* done) { *done = 1; }
 
 __global__ void decim_gain_kernel(const double* __restrict__ y, size_t y_stride, long long n,
                                   int nch, double g_start, double g_step, int apply,
@@ -495,13 +506,24 @@ struct dsdgpu_decim_state {
   // delay lines
   enum { kFresh, kTail, kLines } from = kFresh;
   bool ragged = false;
+  // Calls captured into a graph run later and more than once, so they may not
+  // rest on what the host knows of the stream: from the first one on, every
+  // call takes the stages, whose whole state is the delay lines, and a device
+  // word says whether these are valid yet (see to_lines).
+  bool on_device = false;
+  bool capturing = false;       // this call is captured
+  int* d_done = nullptr;
+  bool buf_in_graph = false;    // a captured call has named d_buf
+  std::vector<double*> old_bufs;
   uint8_t* tail() const { return d_tail + (size_t)tail_buf * nch * tail_cap; }
   ~dsdgpu_decim_state() {
+    if (d_done) cudaFree(d_done);
     if (d_taps) cudaFree(d_taps);
     if (d_tail) cudaFree(d_tail);
     if (d_lut) cudaFree(d_lut);
     if (d_dly) cudaFree(d_dly);
     if (d_buf) cudaFree(d_buf);
+    for (double* b : old_bufs) cudaFree(b);
   }
 };
 
@@ -533,7 +555,7 @@ int launch_decim_f64_fresh(const double* in, size_t in_stride, long long count, 
     const long long m = cur / 2;
     if (m > 0)
       decim_stage_kernel<<<nb(m * nch, 256), 256, 0, st>>>(nz, x, xs, m, zero_dly, pp[k & 1], row,
-                                                           nch);
+                                                           nch, nullptr);
     x = pp[k & 1];
     xs = row;
     cur = m;
@@ -550,22 +572,37 @@ int launch_decim_f64_fresh(const double* in, size_t in_stride, long long count, 
 
 namespace {
 
+// The stages' rows.  Calls that took the product have not allocated them, so the
+// first captured call may have to: allowed in this thread's relaxed mode.  Rows
+// that a graph may name, or that a captured call outgrows, are kept until the
+// state goes.
 int ensure_rows(dsdgpu_context_t* c, dsdgpu_decim_state* s, size_t count) {
   const size_t row = ((count / 2 + 1) + 31) & ~(size_t)31;
-  if (s->row >= row) return DSDGPU_OK;
-  if (s->d_buf) cudaFree(s->d_buf);
+  if (s->row >= row) {
+    s->buf_in_graph |= s->capturing;
+    return DSDGPU_OK;
+  }
+  if (s->d_buf && (s->buf_in_graph || s->capturing)) s->old_bufs.push_back(s->d_buf);
+  else if (s->d_buf) cudaFree(s->d_buf);
   s->d_buf = nullptr;
   s->row = 0;
-  if (cudaMalloc(&s->d_buf, sizeof(double) * 2 * row * (size_t)s->nch) != cudaSuccess)
-    return c->cuda_fail(cudaGetLastError(), "decimation buffers");
+  s->buf_in_graph = s->capturing;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaMalloc(&s->d_buf, sizeof(double) * 2 * row * (size_t)s->nch);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return c->cuda_fail(e, "decimation buffers");
+  }
   s->row = row;
   return DSDGPU_OK;
 }
 
 // `count` decisions through the stages and their delay lines; the last
-// stage's outputs in *y (rows of s->row), *m of them.
+// stage's outputs in *y (rows of s->row), *m of them.  Nothing where *done is set.
 int staged(dsdgpu_context_t* c, dsdgpu_decim_state* s, const uint8_t* d_bits, size_t bits_stride,
-           size_t count, const double** y, size_t* m_out) {
+           size_t count, const double** y, size_t* m_out, const int* done = nullptr) {
   const int nch = s->nch;
   cudaStream_t st = c->stream;
   const int rc = ensure_rows(c, s, count);
@@ -580,12 +617,12 @@ int staged(dsdgpu_context_t* c, dsdgpu_decim_state* s, const uint8_t* d_bits, si
     if (m > 0) {
       if (k == 0) {
         decim_bits_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, s->d_lut, s->taps.h[kDecTaps / 2], d_bits,
-                                                            bits_stride, m, dly, out, s->row, nch);
-        decim_dly_kernel<true><<<nch, 64, 0, st>>>(d_bits, nullptr, bits_stride, 2 * m, dly, nch);
+                                                            bits_stride, m, dly, out, s->row, nch, done);
+        decim_dly_kernel<true><<<nch, 64, 0, st>>>(d_bits, nullptr, bits_stride, 2 * m, dly, nch, done);
       } else {
         decim_stage_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, in, s->row, m, dly, out, s->row,
-                                                             nch);
-        decim_dly_kernel<false><<<nch, 64, 0, st>>>(nullptr, in, s->row, 2 * m, dly, nch);
+                                                             nch, done);
+        decim_dly_kernel<false><<<nch, 64, 0, st>>>(nullptr, in, s->row, 2 * m, dly, nch, done);
       }
       c->launches += 2;
     }
@@ -597,20 +634,45 @@ int staged(dsdgpu_context_t* c, dsdgpu_decim_state* s, const uint8_t* d_bits, si
   return DSDGPU_OK;
 }
 
+// Whether this call is captured; from then on the stream's state is on the device.
+void look_for_capture(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(c->stream, &cap);
+  s->capturing = cap != cudaStreamCaptureStatusNone;
+  if (s->capturing) s->on_device = true;
+}
+
 // The stages' delay lines as the calls so far leave them: zero at a stream's
 // start, else the stages run over the tail from rest.  The tail starts on a
 // whole block and is 64 blocks long (or the whole stream), which is longer
 // than any line's window, so its last values are the same as in one run.
+// A captured call carries these launches into its graph, and they have to run
+// once, whichever of the graph's replays and of the calls after it comes first:
+// they look at *d_done, which the first of them sets.
 int to_lines(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
   if (s->from == dsdgpu_decim_state::kLines) return DSDGPU_OK;
-  cudaMemsetAsync(s->d_dly, 0, sizeof(double) * (size_t)s->stages * s->nch * (kDecTaps - 1), c->stream);
+  const int lines = s->stages * s->nch * (kDecTaps - 1);
+  const int* done = s->on_device ? s->d_done : nullptr;
+  if (done) {
+    decim_rest_kernel<<<std::min(nb(lines, 256), 64u), 256, 0, c->stream>>>(s->d_dly, lines, done);
+    c->launches++;
+  } else {
+    cudaMemsetAsync(s->d_dly, 0, sizeof(double) * (size_t)lines, c->stream);
+  }
   if (s->from == dsdgpu_decim_state::kTail && s->tail_len > 0) {
     const double* y = nullptr;
     size_t m = 0;
-    const int rc = staged(c, s, s->tail(), (size_t)s->tail_cap, (size_t)s->tail_len, &y, &m);
+    const int rc = staged(c, s, s->tail(), (size_t)s->tail_cap, (size_t)s->tail_len, &y, &m, done);
     if (rc) return rc;
   }
+  if (done) {
+    decim_done_kernel<<<1, 1, 0, c->stream>>>(s->d_done);
+    c->launches++;
+  }
+  if (s->capturing) return DSDGPU_OK;   // as far as the host knows, it has not run
   s->from = dsdgpu_decim_state::kLines;
+  s->ragged = false;
+  s->tail_len = 0;
   return DSDGPU_OK;
 }
 
@@ -651,8 +713,10 @@ int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d
   const double step = n > 1 ? (gain_end - gs) / (double)(n - 1) : 0.0;
 
   const MmaPlan& M = s->mma;
-  const bool stages = s->from == dsdgpu_decim_state::kLines || s->ragged;   // at the start of the call
-  const bool all = stages && count < (size_t)128 * M.B;                     // and to its end
+  look_for_capture(c, s);
+  // stages at the start of the call, and to its end
+  const bool stages = s->from == dsdgpu_decim_state::kLines || s->ragged || s->on_device;
+  const bool all = stages && (s->on_device || count < (size_t)128 * M.B);
   const size_t in_row = d_dop ? count / 16 * sizeof(float) : count;
   const size_t in_step = d_dop ? stride * sizeof(float) : stride;
   if (!all && n > 0 &&
@@ -681,8 +745,6 @@ int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d
   if (stages) {
     int rc = to_lines(c, s);
     if (rc) return rc;
-    s->ragged = false;
-    s->tail_len = 0;
     const size_t part = all ? count : (size_t)64 * M.B;
     const uint8_t* bits = d_bits;
     size_t bstride = stride;
@@ -778,7 +840,8 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
   s->tail_cap = 65 * s->mma.B;
   if (cudaMalloc(&s->d_dly, dbytes) != cudaSuccess || cudaMalloc(&s->d_lut, sizeof lut) != cudaSuccess ||
       cudaMalloc(&s->d_taps, taps.size() * sizeof(uint32_t)) != cudaSuccess ||
-      cudaMalloc(&s->d_tail, (size_t)2 * nch * s->tail_cap) != cudaSuccess) {
+      cudaMalloc(&s->d_tail, (size_t)2 * nch * s->tail_cap) != cudaSuccess ||
+      cudaMalloc(&s->d_done, sizeof(int)) != cudaSuccess) {
     delete s;
     return c->cuda_fail(cudaGetLastError(), "decimation buffers");
   }
@@ -796,6 +859,7 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
   cudaMemcpyAsync(s->d_lut, lut, sizeof lut, cudaMemcpyHostToDevice, c->stream);
   cudaMemcpyAsync(s->d_taps, taps.data(), taps.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
   cudaMemsetAsync(s->d_dly, 0, dbytes, c->stream);
+  cudaMemsetAsync(s->d_done, 0, sizeof(int), c->stream);
   decim_free(c->decim);
   c->decim = s;
   return c->check_status();
@@ -804,11 +868,19 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
 int dsdgpu_decim_reset(dsdgpu_context_t* c) {
   if (!c) return DSDGPU_ERR_ARG;
   if (!c->decim) return c->fail(DSDGPU_ERR_STATE, "decimation not set up");
-  // nothing on the device has to change: the next call starts from no history
-  c->decim->from = dsdgpu_decim_state::kFresh;
-  c->decim->tail_len = 0;
-  c->decim->ragged = false;
-  return DSDGPU_OK;
+  dsdgpu_decim_state* s = c->decim;
+  s->tail_len = 0;
+  s->ragged = false;
+  s->from = dsdgpu_decim_state::kFresh;
+  // nothing on the device has to change (the next call starts from no history),
+  // unless a graph may run next
+  if (!s->on_device) return DSDGPU_OK;
+  cudaSetDevice(c->device);
+  cudaMemsetAsync(s->d_dly, 0, sizeof(double) * (size_t)s->stages * s->nch * (kDecTaps - 1), c->stream);
+  decim_done_kernel<<<1, 1, 0, c->stream>>>(s->d_done);
+  c->launches++;
+  s->from = dsdgpu_decim_state::kLines;
+  return c->check_status();
 }
 
 int dsdgpu_decim_process_async(dsdgpu_context_t* c, int nch, const uint8_t* d_bits,
@@ -835,10 +907,9 @@ int dsdgpu_decim_process_f64_async(dsdgpu_context_t* c, int nch, const double* d
     return c->fail(DSDGPU_ERR_ARG, "row stride shorter than the count");
   cudaSetDevice(c->device);
   cudaStream_t st = c->stream;
+  look_for_capture(c, s);
   int rc = to_lines(c, s);
   if (rc) return rc;
-  s->ragged = false;
-  s->tail_len = 0;
   rc = ensure_rows(c, s, count);
   if (rc) return rc;
   double* buf[2] = {s->d_buf, s->d_buf + s->row * (size_t)nch};
@@ -850,8 +921,9 @@ int dsdgpu_decim_process_f64_async(dsdgpu_context_t* c, int nch, const double* d
     double* out = buf[k & 1];
     double* dly = s->d_dly + (size_t)k * nch * (kDecTaps - 1);
     if (m > 0) {
-      decim_stage_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, in, istride, m, dly, out, s->row, nch);
-      decim_dly_kernel<false><<<nch, 64, 0, st>>>(nullptr, in, istride, 2 * m, dly, nch);
+      decim_stage_kernel<<<nb(m * nch, 256), 256, 0, st>>>(s->nz, in, istride, m, dly, out, s->row, nch,
+                                                           nullptr);
+      decim_dly_kernel<false><<<nch, 64, 0, st>>>(nullptr, in, istride, 2 * m, dly, nch, nullptr);
       c->launches += 2;
     }
     in = out;

@@ -230,3 +230,71 @@ def test_decim_in_place(oracle, fs_in, fs_out, nch):
         assert torch.equal(raw.view(torch.float32)[:, :n], want), frames
     for h in hs:
         L.dsdgpu_destroy(h)
+
+
+@pytest.mark.parametrize("before", ["fresh", "blocks", "ragged", "stages"])
+@pytest.mark.parametrize("live_first", [False, True])
+def test_decim_captured_calls(oracle, before, live_first):
+    """A captured dsdgpu_decim_process_async continues the stream at every
+    replay of its graph, whatever the stream was before the capture, mixed with
+    plain calls after it, and from rest after a reset."""
+    from foo_dsd_trellis_gb300 import _lib
+    fs_in, fs_out, nch, D = 5644800, 176400, 2, 32
+    rng = np.random.default_rng(len(before))
+    L, rt = _lib.load(), C.CDLL("libcudart.so.13")
+    h, st = C.c_void_p(), C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    _lib.check(h, L.dsdgpu_decim_setup(h, fs_in, fs_out, nch))
+    _lib.check(h, L.dsdgpu_get_stream(h, C.byref(st)))
+    refs = [oracle.Decimator(fs_in, fs_out) for _ in range(nch)]
+    cap = 300 * D
+
+    def bits(n):
+        b = (rng.random((nch, cap)) > 0.4).astype(np.uint8)
+        return b, torch.from_numpy(b).cuda()
+
+    def check(out, b, n):
+        L.dsdgpu_synchronize(h)
+        for c in range(nch):
+            want = refs[c].process(b[c, :n].astype(np.float64) * 2 - 1).astype(np.float32)
+            np.testing.assert_allclose(out.cpu().numpy()[c, : len(want)], want, rtol=0, atol=2e-7)
+
+    def call(d_in, d_out, n):
+        m = C.c_size_t()
+        torch.cuda.synchronize()
+        _lib.check(h, L.dsdgpu_decim_process_async(h, nch, d_in.data_ptr(), cap, n, d_out.data_ptr(),
+                                                   cap // D, 1.0, 1.0, C.byref(m)))
+
+    out = torch.zeros((nch, cap // D), dtype=torch.float32, device="cuda")
+    for n in {"fresh": [], "blocks": [200 * D, 70 * D], "ragged": [200 * D + 5], "stages": [200 * D + 5, 7]}[before]:
+        b, d = bits(n)
+        call(d, out, n)
+        check(out, b, n)
+    n_cap = 150 * D + 9
+    _, d_in = bits(n_cap)
+    d_out = torch.zeros_like(out)
+    graph, ex = C.c_void_p(), C.c_void_p()
+    torch.cuda.synchronize()
+    assert rt.cudaStreamBeginCapture(st, 1) == 0
+    call_rc = L.dsdgpu_decim_process_async(h, nch, d_in.data_ptr(), cap, n_cap, d_out.data_ptr(), cap // D,
+                                           1.0, 1.0, C.byref(C.c_size_t()))
+    assert rt.cudaStreamEndCapture(st, C.byref(graph)) == 0 and call_rc == 0
+    assert rt.cudaGraphInstantiate(C.byref(ex), graph, C.c_ulonglong(0)) == 0
+    for what in (["live"] if live_first else []) + ["replay", "replay", "live", "replay", "reset", "replay", "live"]:
+        if what == "reset":
+            _lib.check(h, L.dsdgpu_decim_reset(h))
+            refs = [oracle.Decimator(fs_in, fs_out) for _ in range(nch)]
+            continue
+        if what == "live":
+            b, d = bits(0)
+            call(d, out, 290 * D)
+            check(out, b, 290 * D)
+        else:
+            b, d = bits(0)
+            d_in.copy_(d)
+            torch.cuda.synchronize()
+            assert rt.cudaGraphLaunch(ex, st) == 0
+            check(d_out, b, n_cap)
+    rt.cudaGraphExecDestroy(ex)
+    rt.cudaGraphDestroy(graph)
+    L.dsdgpu_destroy(h)
