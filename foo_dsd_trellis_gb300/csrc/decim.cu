@@ -36,7 +36,9 @@
 // factor: a call whose length is not a multiple of D drops inputs at some
 // stage, and what follows is no longer one filter over the decisions.  The
 // next call's first outputs (those whose window reaches back over that point)
-// and calls shorter than 128 B then take this form; so do FP64 inputs.  IPP's
+// and calls shorter than 128 B then take this form; so do FP64 inputs, captured
+// calls, ragged streams up to the sizes of kRaggedFrom and one stage alone from
+// kOneStageFrom.  IPP's
 // summation order and use of FMA are not known, so the stages take the
 // cheapest exact-enough form:
 //   * the 63-tap half-band's taps at odd k other than the centre are the
@@ -678,6 +680,19 @@ int to_lines(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
 
 }  // namespace
 
+// Decisions of a call (over all channels) from which the product pays though it
+// costs more launches than the stages, by the number of stages: a ragged call of
+// a stream whose last one was ragged too, which would run the tail through the
+// stages (a launch costs 4.9 us here) to get the first outputs.  Measured, calls
+// of one length, 1 / 2 / 6 channels alike, us by stages alone / with the
+// product: 4 stages 1.0 M decisions 95 / 110, 2.0 M 129 / 117; 7 stages 20 k
+// 94 / 168, 2.5 M 184 / 186, 4.0 M 234 / 185; 9 stages 4.0 M 254 / 250.
+constexpr double kRaggedFrom[] = {0, 0.5e6, 4.0e6, 2.0e6, 1.8e6, 2.0e6, 2.2e6, 2.6e6, 3.1e6, 4.0e6};
+static_assert(sizeof kRaggedFrom / sizeof(double) == kMaxStages + 1, "one for every number of stages");
+// One stage (a product tile for every output of a block, eight of them): also
+// the calls that follow whole blocks; 0.5 M decisions 27 / 34 us, 6.0 M 83 / 214.
+constexpr double kOneStageFrom = 0.5e6;
+
 // Whether [a, a + na) and [b, b + nb) share a byte.
 static bool overlap(const void* a, size_t na, const void* b, size_t nb) {
   const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
@@ -714,9 +729,12 @@ int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d
 
   const MmaPlan& M = s->mma;
   look_for_capture(c, s);
+  const int rag = (int)(count % (size_t)M.B);
+  const double work = (double)count * nch;
   // stages at the start of the call, and to its end
-  const bool stages = s->from == dsdgpu_decim_state::kLines || s->ragged || s->on_device;
-  const bool all = stages && (s->on_device || count < (size_t)128 * M.B);
+  const bool only = s->on_device || (s->stages == 1 && work >= kOneStageFrom);
+  const bool stages = s->from == dsdgpu_decim_state::kLines || s->ragged || only;
+  const bool all = only || (stages && (count < (size_t)128 * M.B || (rag && work < kRaggedFrom[s->stages])));
   const size_t in_row = d_dop ? count / 16 * sizeof(float) : count;
   const size_t in_step = d_dop ? stride * sizeof(float) : stride;
   if (!all && n > 0 &&
@@ -779,7 +797,6 @@ int decim_run(dsdgpu_context_t* c, int nch, const float* d_dop, const uint8_t* d
   I.tail = s->tail();
   I.tail_len = s->tail_len;
   I.tail_stride = (size_t)s->tail_cap;
-  const int rag = (int)(count % (size_t)M.B);
   const long long total = (long long)s->tail_len + (long long)count;
   const int keep = (int)std::min<long long>(total, 64ll * M.B + rag);
   uint8_t* next = s->d_tail + (size_t)(s->tail_buf ^ 1) * nch * s->tail_cap;

@@ -298,3 +298,59 @@ def test_decim_captured_calls(oracle, before, live_first):
     rt.cudaGraphExecDestroy(ex)
     rt.cudaGraphDestroy(graph)
     L.dsdgpu_destroy(h)
+
+
+@pytest.mark.parametrize("fs_in,fs_out,n", [(2822400, 1411200, 60001), (2822400, 176400, 2053),
+                                            (5644800, 44100, 20001), (22579200, 44100, 65537),
+                                            (5644800, 44100, 400000 + 5)])
+def test_decim_ragged_calls_launch_no_more_than_the_stages(oracle, fs_in, fs_out, n):
+    """A stream whose every call ends inside a block, in calls long enough for
+    the matrix product (128 blocks and more): from the second on a call takes at
+    most the stages' launches, and the outputs stay the oracle's."""
+    from foo_dsd_trellis_gb300 import _lib
+    nch, S = 2, (fs_in // fs_out).bit_length() - 1
+    rng = np.random.default_rng(n)
+    L = _lib.load()
+    h = C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    _lib.check(h, L.dsdgpu_decim_setup(h, fs_in, fs_out, nch))
+    refs = [oracle.Decimator(fs_in, fs_out) for _ in range(nch)]
+    out = torch.zeros((nch, n), dtype=torch.float32, device="cuda")
+    count = []
+    for k in range(5):
+        bits = (rng.random((nch, n)) > 0.4).astype(np.uint8)
+        d = torch.from_numpy(bits).cuda()
+        m, v0, v1 = C.c_size_t(), C.c_uint64(), C.c_uint64()
+        L.dsdgpu_launch_count(h, C.byref(v0))
+        _lib.check(h, L.dsdgpu_decim_process(h, nch, d.data_ptr(), n, n, out.data_ptr(), n, 1.0, 1.0,
+                                             C.byref(m)))
+        L.dsdgpu_launch_count(h, C.byref(v1))
+        count.append(v1.value - v0.value)
+        for c in range(nch):
+            want = refs[c].process(bits[c].astype(np.float64) * 2 - 1)
+            assert m.value == len(want)
+            np.testing.assert_allclose(out[c, : m.value].cpu().numpy(), want, rtol=0, atol=2e-7)
+    assert max(count[2:]) <= 2 * S + 1, count
+    L.dsdgpu_destroy(h)
+
+
+def test_decim_one_stage_long_and_short_calls(oracle):
+    """Ratio 2, where long calls take the stages and short ones the product:
+    a stream of both."""
+    from foo_dsd_trellis_gb300 import _lib
+    nch = 1
+    L = _lib.load()
+    h = C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    _lib.check(h, L.dsdgpu_decim_setup(h, 2822400, 1411200, nch))
+    ref = oracle.Decimator(2822400, 1411200)
+    rng = np.random.default_rng(3)
+    for n in (600, 16 * 33000, 600, 16 * 33000 + 3, 5000, 499984, 500000):
+        bits = (rng.random(n) > 0.4).astype(np.uint8)
+        d, out, m = torch.from_numpy(bits).cuda(), torch.zeros(n, device="cuda"), C.c_size_t()
+        _lib.check(h, L.dsdgpu_decim_process(h, nch, d.data_ptr(), n, n, out.data_ptr(), n, 1.0, 1.0,
+                                             C.byref(m)))
+        want = ref.process(bits.astype(np.float64) * 2 - 1)
+        assert m.value == len(want)
+        np.testing.assert_allclose(out[: m.value].cpu().numpy(), want, rtol=0, atol=2e-7, err_msg=str(n))
+    L.dsdgpu_destroy(h)
