@@ -425,63 +425,79 @@ __host__ size_t mma_smem_bytes(const MmaPlan& M) {
          sizeof(float) * (size_t)kMmaDigits * 16 * kAccRow + sizeof(int) * kMmaDigits * kMmaCols;
 }
 
-// The plan of `stages` stages and its taps in the order of the A fragments:
-// [phase][digit][16-lag group][step][lane][4 registers of two bf16].
-std::vector<uint32_t> mma_taps(int stages, const DecNz& nz, MmaPlan* M) {
+// The plan of `stages` stages (all but its shift, which the taps' peak decides).
+int mma_len(int stages) { return 62 * ((1 << stages) - 1) + 1; }
+size_t mma_words(const MmaPlan& M) { return (size_t)M.F * kMmaDigits * M.T * (M.B / 16) * 32 * 4; }
+MmaPlan mma_plan(int stages) {
   const int D = 1 << stages;
-  M->B = D < 16 ? 16 : D;
-  M->F = M->B / D;
-  // the stages' combined response: stage k's taps 2^k inputs apart
-  std::vector<double> h(1, 1.0);
-  for (int k = 0; k < stages; k++) {
-    const int gap = 1 << k;
-    std::vector<double> n(h.size() + (size_t)62 * gap, 0.0);
-    for (size_t i = 0; i < h.size(); i++)
-      for (int q = 0; q < kNzTaps; q++) n[i + (size_t)nz.k[q] * gap] += h[i] * nz.h[q];
-    h.swap(n);
+  MmaPlan M{};
+  M.B = D < 16 ? 16 : D;
+  M.F = M.B / D;
+  const int J = (mma_len(stages) - 1 + M.B - 1) / M.B + 1;
+  M.T = (J + 15) / 16;
+  return M;
+}
+
+// The plan's taps, formed on the device: on the host they took 1.8 ms of a
+// setup at ratio 512.  One stage's taps, `gap` inputs apart, times the response
+// of the stages before it, h of `len` taps (nullptr: the unit impulse):
+__global__ void decim_conv_kernel(const __grid_constant__ DecNz T, const double* __restrict__ h, int len,
+                                  int gap, double* __restrict__ out) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= len + 62 * gap) return;
+  double acc = 0.0;
+  for (int q = kNzTaps - 1; q >= 0; q--) {
+    const int i = j - T.k[q] * gap;
+    if (i >= 0 && i < len) acc = __dadd_rn(acc, __dmul_rn(h ? h[i] : 1.0, T.h[q]));
   }
-  const long long last = (long long)h.size() - 1;
-  const int J = (int)((last + M->B - 1) / M->B) + 1;
-  M->T = (J + 15) / 16;
-  double peak = 0.0;
-  for (double v : h) peak = std::max(peak, std::fabs(v));
-  M->shift = 61;
-  while (std::ldexp(peak, M->shift) > std::ldexp(1.0, 54)) M->shift--;
-  const int KS = M->B / 16, steps = M->T * KS;
-  std::vector<uint32_t> out((size_t)M->F * kMmaDigits * steps * 32 * 4, 0u);
-  auto bf16 = [](int v) {   // |v| <= 128: exact
-    float f = (float)v;
-    uint32_t u;
-    memcpy(&u, &f, 4);
-    return u >> 16;
-  };
-  std::vector<int8_t> dig(h.size() * kMmaDigits);
-  for (size_t i = 0; i < h.size(); i++) {
-    long long v = std::llrint(std::ldexp(h[i], M->shift));
-    for (int k = 0; k < kMmaDigits; k++) {   // balanced digits, -128 .. 127
-      int d = (int)(v & 255);
-      if (d > 127) d -= 256;
-      dig[i * kMmaDigits + k] = (int8_t)d;
+  out[j] = acc;
+}
+
+__global__ void __launch_bounds__(1024) decim_peak_kernel(const double* __restrict__ h, int len,
+                                                          double* __restrict__ peak) {
+  __shared__ double part[32];
+  double m = 0.0;
+  for (int i = threadIdx.x; i < len; i += blockDim.x) m = fmax(m, fabs(h[i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = part[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) *peak = m;
+  }
+}
+
+// the taps in the order of the A fragments:
+// [phase][digit][16-lag group][step][lane][4 registers of two bf16]
+__global__ void decim_frag_kernel(const MmaPlan M, int D, const double* __restrict__ h, int len, double one,
+                                  unsigned* __restrict__ out, int words) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= words) return;
+  const int r = w & 3, lane = (w >> 2) & 31, KS = M.B / 16;
+  int at = w >> 7;
+  const int ks = at % KS;
+  at /= KS;
+  const int t = at % M.T;
+  at /= M.T;
+  const int k = at % kMmaDigits, ph = at / kMmaDigits;
+  const int row = lane / 4 + (r & 1) * 8;
+  unsigned word = 0;
+  for (int e = 0; e < 2; e++) {
+    const int kk = 2 * (lane % 4) + e + (r >> 1) * 8;
+    const int tap = D * ph + M.B * (16 * t + row) - (16 * ks + kk);
+    if (tap < 0 || tap >= len) continue;
+    long long v = __double2ll_rn(h[tap] * one);   // the product is exact
+    int d = 0;
+    for (int i = 0; i <= k; i++) {                // balanced digits, -128 .. 127
+      d = (int)(signed char)(v & 255);
       v = (v - d) >> 8;
     }
+    word |= (__float_as_uint((float)d) >> 16) << (16 * e);   // bf16: exact
   }
-  for (int ph = 0; ph < M->F; ph++)
-    for (int k = 0; k < kMmaDigits; k++)
-      for (int t = 0; t < M->T; t++)
-        for (int ks = 0; ks < KS; ks++)
-          for (int lane = 0; lane < 32; lane++)
-            for (int r = 0; r < 4; r++) {
-              uint32_t w = 0;
-              for (int e = 0; e < 2; e++) {
-                const int row = lane / 4 + (r & 1) * 8;
-                const int kk = 2 * (lane % 4) + e + (r >> 1) * 8;
-                const long long tap = (long long)D * ph + (long long)M->B * (16 * t + row) - (16 * ks + kk);
-                const int d = tap >= 0 && tap <= last ? dig[(size_t)tap * kMmaDigits + k] : 0;
-                w |= bf16(d) << (16 * e);
-              }
-              out[((((size_t)ph * kMmaDigits + k) * steps + (size_t)t * KS + ks) * 32 + lane) * 4 + r] = w;
-            }
-  return out;
+  out[w] = word;
 }
 
 unsigned nb(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -598,6 +614,34 @@ int ensure_rows(dsdgpu_context_t* c, dsdgpu_decim_state* s, size_t count) {
     return c->cuda_fail(e, "decimation buffers");
   }
   s->row = row;
+  return DSDGPU_OK;
+}
+
+// The whole-chain form's taps in s->d_taps, and the plan's shift.
+int form_taps(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
+  const int len = mma_len(s->stages), words = (int)mma_words(s->mma);
+  const int rc = c->ensure_scratch(sizeof(double) * (2 * (size_t)len + 1));
+  if (rc) return rc;
+  double* buf[2] = {(double*)c->d_scratch, (double*)c->d_scratch + len};
+  double* d_peak = buf[1] + len;
+  const double* h = nullptr;
+  for (int k = 0; k < s->stages; k++) {
+    const int n = mma_len(k + 1);
+    decim_conv_kernel<<<nb(n, 128), 128, 0, c->stream>>>(s->nz, h, mma_len(k), 1 << k, buf[k & 1]);
+    h = buf[k & 1];
+  }
+  decim_peak_kernel<<<1, 1024, 0, c->stream>>>(h, len, d_peak);
+  double peak = 0.0;
+  cudaMemcpyAsync(&peak, d_peak, sizeof peak, cudaMemcpyDeviceToHost, c->stream);
+  const cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (e != cudaSuccess) return c->cuda_fail(e, "decimation taps");
+  // the digits' sum stays below 2^63 (sum |h| < 1.9), a tap below 2^54
+  s->mma.shift = 61;
+  while (std::ldexp(peak, s->mma.shift) > std::ldexp(1.0, 54)) s->mma.shift--;
+  decim_frag_kernel<<<nb(words, 256), 256, 0, c->stream>>>(s->mma, 1 << s->stages, h, len,
+                                                           std::ldexp(1.0, s->mma.shift), (unsigned*)s->d_taps,
+                                                           words);
+  c->launches += s->stages + 2;
   return DSDGPU_OK;
 }
 
@@ -853,10 +897,10 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
       lut[g * 256 + p] = acc;
     }
   const size_t dbytes = sizeof(double) * (size_t)S * nch * (kDecTaps - 1);
-  const std::vector<uint32_t> taps = mma_taps(S, s->nz, &s->mma);
+  s->mma = mma_plan(S);
   s->tail_cap = 65 * s->mma.B;
   if (cudaMalloc(&s->d_dly, dbytes) != cudaSuccess || cudaMalloc(&s->d_lut, sizeof lut) != cudaSuccess ||
-      cudaMalloc(&s->d_taps, taps.size() * sizeof(uint32_t)) != cudaSuccess ||
+      cudaMalloc(&s->d_taps, mma_words(s->mma) * sizeof(uint32_t)) != cudaSuccess ||
       cudaMalloc(&s->d_tail, (size_t)2 * nch * s->tail_cap) != cudaSuccess ||
       cudaMalloc(&s->d_done, sizeof(int)) != cudaSuccess) {
     delete s;
@@ -874,7 +918,11 @@ int dsdgpu_decim_setup(dsdgpu_context_t* c, unsigned fs_in, unsigned fs_out, int
     return c->cuda_fail(cudaGetLastError(), "decimation kernel attributes");
   }
   cudaMemcpyAsync(s->d_lut, lut, sizeof lut, cudaMemcpyHostToDevice, c->stream);
-  cudaMemcpyAsync(s->d_taps, taps.data(), taps.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
+  const int rc = form_taps(c, s);
+  if (rc) {
+    delete s;
+    return rc;
+  }
   cudaMemsetAsync(s->d_dly, 0, dbytes, c->stream);
   cudaMemsetAsync(s->d_done, 0, sizeof(int), c->stream);
   decim_free(c->decim);
