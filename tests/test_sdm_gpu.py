@@ -528,3 +528,73 @@ def test_products_in_and_out_of_range(oracle, K, order, njobs):
             want = oracle.sdm_bits(refs[c], rows[row, :n])
             for i in np.flatnonzero(((idx < half) == fresh) & (idx % 4 == row))[::29]:
                 np.testing.assert_array_equal(got[i].cpu().numpy(), want, err_msg=f"{c} {n} {i}")
+
+
+def _filter(kind, order):
+    """A filter of the table; "odd": the table's odd orders above DSD512, whose
+    odd g are zero; "g0": every resonator at 0; "trained": every g nonzero;
+    "cut": a table filter truncated or zero-padded to `order`."""
+    if kind == "odd":
+        return _ntf({5: "sdm-5", 7: "sdm-7"}[order], 45158400)
+    src = (_ntf("clans-4", 2822400) if order <= 4 else _ntf("clans-8", 11289600)) if kind == "cut" else \
+        _ntf({5: "clans-5", 6: "clans-6", 7: "clans-7", 8: "clans-8"}[order], 5644800)
+
+    class F:
+        pass
+    f = F()
+    f.order, f.a, f.g = order, [0.0] * order, [0.0] * order
+    m = min(order, src.order)
+    f.a[:m], f.g[:m] = list(src.a[:m]), list(src.g[:m])
+    if kind == "g0":
+        f.g = [0.0] * order
+    if kind == "trained":
+        f.g = [v + 1e-5 * (i + 1) for i, v in enumerate(f.g)]
+    return f
+
+
+@pytest.mark.parametrize("kind,order", [("odd", 7), ("odd", 5), ("g0", 6), ("g0", 7), ("trained", 7),
+                                        ("trained", 8), ("cut", 2), ("cut", 3), ("cut", 9), ("cut", 10)])
+@pytest.mark.parametrize("K,lanes", [(32, 0), (19, 0), (16, 16), (7, 8)])
+def test_warp_kernel_filters(oracle, kind, order, K, lanes):
+    """The warp kernels with filters whose coefficients the integer products do
+    not take (a zero a, a zero g where the table has none), with the other
+    pattern of zero g and with none: streamed, equal to the oracle."""
+    from foo_dsd_trellis_gb300 import _lib
+    f = _filter(kind, order)
+    depth, lat = 40, 48
+    n = 2600
+    x = 0.5 * multitone(n, seed=order + K)
+    x[700:900] = 0.0
+    ref = _ora(oracle, f, depth, K, lat)
+    g = _gpu_sdm(f, depth, K, lat)
+    if lanes:
+        g.set_option(_lib.OPT_SDM_LANES, lanes)
+    for lo, hi in ((0, 31), (31, 1500), (1500, n)):
+        got = g.process_block(torch.from_numpy(x[lo:hi].copy()).cuda())[0].cpu().numpy()
+        np.testing.assert_array_equal(got, oracle.sdm_bits(ref, x[lo:hi]))
+    assert g.last_sdm_kernel() == f"sdm_jobs_kernel<{order},{lanes or 32}>"
+    info, q = ref.info(), g.query(0)
+    assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
+        (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"])
+    np.testing.assert_array_equal(q["best_state"], ref.best_state())
+
+
+@pytest.mark.parametrize("kind,order", [("table", 7), ("odd", 7), ("g0", 6)])
+def test_parts_kernel_filters(kind, order):
+    """The balanced launch (jobs in queued parts) equals one job a warp for the
+    same filters."""
+    from foo_dsd_trellis_gb300 import _lib
+    from foo_dsd_trellis_gb300.das import DasChannels
+    f = _filter(kind, order)
+    pipes = 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    S = (pipes + pipes // 20) // 2 + 1            # segments per channel, 2 channels
+    x = np.stack([multitone(S * 9000, 30 + c) * 0.5 for c in range(2)])
+    fir = torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    outs = []
+    for balance in (1, 0):
+        d = DasChannels(f.order, f.a, f.g, 16, 32, 32, num_channels=2)
+        _lib.check(d.h, d.L.dsdgpu_set_option(d.h, _lib.OPT_SDM_BALANCE, balance))
+        outs.append(d.process_chunk(fir, nsegs=S, seed_mode=0)[0])
+        assert d.last_sdm_kernel().startswith("sdm_parts_kernel" if balance else "sdm_jobs_kernel")
+        d.close()
+    assert torch.equal(outs[0], outs[1])
