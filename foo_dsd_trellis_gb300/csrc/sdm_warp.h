@@ -303,10 +303,7 @@ __device__ __forceinline__ void word_sort(unsigned& c0, unsigned& c1, int lane, 
   }
 }
 
-// The same order by the whole (key, index) pairs, for the samples whose words
-// do not tell (two children within 2^-21 of each other's cost, a cost out of
-// the words' range, or one that is not finite).  Not unrolled: it is rare, and
-// its code stays out of the step loop's registers.
+// The same order by the whole (key, index) pairs.  Not unrolled: it is rare.
 template <int LPJ>
 __device__ __forceinline__ void full_sort(long long& kA, int& iA, long long& kB, int& iB, int lane,
                                           unsigned hm) {
@@ -333,6 +330,50 @@ __device__ __forceinline__ void full_sort(long long& kA, int& iA, long long& kB,
       }
     }
   }
+}
+
+// The order of the children (this lane's keys k0, k1; LLONG_MAX: no child) for
+// the samples whose words do not tell: two children within 2^-21 of each other's
+// cost, a cost out of the words' range, or one that is not finite.  The words of
+// the keys' distances from the least one tell nearly always, above all once a
+// modulator has run away (its costs agree to many places on every sample, for
+// good); else the whole pairs are sorted.  Out of line: its code stays out of the
+// step loop's registers.  Returns the children at sorted positions 2 * lane and
+// 2 * lane + 1 as bits 0 .. 5 and 6 ..  K = 32, order 7, a signal that overloads
+// the modulator: 5.7 us a step with the pairs' sort alone.
+template <int LPJ>
+static __device__ __noinline__ int order_again(long long k0, long long k1, int lane, unsigned hm) {
+  // the least key and the largest distance from it, of those that are costs
+  const bool c0 = (unsigned long long)k0 < 0x7ff0000000000000ull, c1 = (unsigned long long)k1 < 0x7ff0000000000000ull;
+  const unsigned h0 = c0 ? (unsigned)(k0 >> 32) : ~0u, h1 = c1 ? (unsigned)(k1 >> 32) : ~0u;
+  const unsigned mh = __reduce_min_sync(hm, min(h0, h1));
+  const unsigned ml = __reduce_min_sync(hm, min(h0 == mh ? (unsigned)k0 : ~0u, h1 == mh ? (unsigned)k1 : ~0u));
+  const unsigned long long least = (unsigned long long)mh << 32 | ml;
+  const unsigned long long d0 = c0 ? (unsigned long long)k0 - least : 0ull, d1 = c1 ? (unsigned long long)k1 - least : 0ull;
+  const unsigned rh = __reduce_max_sync(hm, (unsigned)(max(d0, d1) >> 32));
+  const unsigned rl = __reduce_max_sync(hm, rh ? 0u : (unsigned)max(d0, d1));
+  const int bits = rh ? 64 - __clz((int)rh) : 32 - __clz((int)rl);
+  const int shift = bits > 25 ? bits - 25 : 0;
+  unsigned w0 = ((c0 ? (unsigned)(d0 >> shift) : kWordNone) << 6) | (unsigned)(2 * lane);
+  unsigned w1 = ((c1 ? (unsigned)(d1 >> shift) : kWordNone) << 6) | (unsigned)(2 * lane + 1);
+  word_sort<LPJ>(w0, w1, lane, hm, [](int) {});
+  int i0 = (int)(w0 & 63u), i1 = (int)(w1 & 63u);
+  auto key_at = [&](int i) {
+    const long long a = __shfl_sync(hm, k0, i >> 1, LPJ), b = __shfl_sync(hm, k1, i >> 1, LPJ);
+    return (i & 1) ? b : a;
+  };
+  long long s0 = key_at(i0), s1 = key_at(i1);
+  const long long after = __shfl_down_sync(hm, s0, 1, LPJ);
+  const int ia = __shfl_down_sync(hm, i0, 1, LPJ);
+  const bool wrong = key_less(s1, i1, s0, i0) || (lane < LPJ - 1 && key_less(after, ia, s1, i1));
+  if (__any_sync(hm, wrong)) {
+    s0 = k0;
+    s1 = k1;
+    i0 = 2 * lane;
+    i1 = 2 * lane + 1;
+    full_sort<LPJ>(s0, i0, s1, i1, lane, hm);
+  }
+  return i0 | i1 << 6;
 }
 
 // Stages of the bitonic sort of 2 * LPJ keys: log2(2 LPJ) (log2(2 LPJ) + 1) / 2
@@ -599,10 +640,9 @@ __device__ void run_job(const SdmParams& P, const SdmJob& job, SdmCtx* __restric
       const bool same = (c0 >> 6) == (c1 >> 6) && (c1 >> 6) != kWordNone;
       const bool same2 = lane < LPJ - 1 && (c1 >> 6) == (after >> 6) && (c1 >> 6) != kWordNone;
       if (__any_sync(hm, same || same2 || odd_key)) {
-        long long sk0 = live ? key0 : LLONG_MAX, sk1 = live ? key1 : LLONG_MAX;
-        si0 = 2 * lane;
-        si1 = 2 * lane + 1;
-        full_sort<LPJ>(sk0, si0, sk1, si1, lane, hm);
+        const int both = order_again<LPJ>(live ? key0 : LLONG_MAX, live ? key1 : LLONG_MAX, lane, hm);
+        si0 = both & 63;
+        si1 = both >> 6;
       }
     }
     // All candidates carry one traceback bit nearly always (they share their

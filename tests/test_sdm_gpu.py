@@ -598,3 +598,30 @@ def test_parts_kernel_filters(kind, order):
         assert d.last_sdm_kernel().startswith("sdm_parts_kernel" if balance else "sdm_jobs_kernel")
         d.close()
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("K,depth,lanes", [(32, 64, 0), (32, 6, 0), (18, 48, 0), (16, 8, 16), (8, 8, 8), (4, 8, 4),
+                                           (2, 4, 2)])
+@pytest.mark.parametrize("name,rate,amp,odd", [("clans-7", 5644800, 4.0, 0.0), ("sdm-8", 45158400, 0.4, 0.0),
+                                               ("clans-6", 5644800, 0.5, 1e300)])
+def test_runaway_modulator_warp_kernel(oracle, K, depth, lanes, name, rate, amp, odd):
+    """A modulator that has run away (no limiter): its costs leave the range of
+    the sort's words and agree to many places, or are not finite after an input
+    of 1e300; the order then comes from the keys' distances or from the whole
+    keys."""
+    from foo_dsd_trellis_gb300 import _lib
+    f = _ntf(name, rate)
+    x = amp * multitone(2500, seed=K)
+    x[1700] += odd
+    ref = _ora(oracle, f, depth, K, 40)
+    g = _gpu_sdm(f, depth, K, 40)
+    if lanes:
+        g.set_option(_lib.OPT_SDM_LANES, lanes)
+    for lo, hi in ((0, 1000), (1000, 2500)):
+        got = g.process_block(torch.from_numpy(x[lo:hi].copy()).cuda())[0].cpu().numpy()
+        np.testing.assert_array_equal(got, oracle.sdm_bits(ref, x[lo:hi]))
+    assert g.last_sdm_kernel().startswith("sdm_jobs_kernel")
+    info, q = ref.info(), g.query(0)
+    assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
+        (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"])
+    np.testing.assert_array_equal(q["best_state"], ref.best_state())
