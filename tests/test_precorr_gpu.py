@@ -149,3 +149,28 @@ def test_precorr_chunks_that_do_not_stand(oracle, name, limit):
         pos += ln
         got = gpu.process_block(torch.from_numpy(blk).cuda())[0].cpu().numpy()
         np.testing.assert_array_equal(got, ref.process(blk), err_msg=str(pos))
+
+
+@pytest.mark.parametrize("nch", [3, 33])
+def test_precorr_channels_of_one_warp_that_differ(oracle, nch):
+    """Channels side by side of which one meets the limiter at times, one is NaN
+    from some point on, and one has run ahead of the others by a few samples
+    (its first sample is not theirs): each equals the restatement alone."""
+    from foo_dsd_trellis_gb300 import ntf
+    from foo_dsd_trellis_gb300.precorr import PreCorr
+    f, limit, n = ntf.get_filter("clans-7", 5644800), 12.0, 4000
+    rng = np.random.default_rng(nch)
+    x = np.stack([0.4 * multitone(n, 70 + c) for c in range(nch)])
+    x[1, 700:900] *= 30.0
+    x[1, 3000:3020] *= 30.0
+    x[nch - 1, 2000] = np.nan
+    x = x.astype(np.float32).astype(np.float64)
+    ahead = (0.3 * rng.standard_normal(5)).astype(np.float32).astype(np.float64)
+    gpu = PreCorr(f.order, f.a, f.g, limit, num_channels=nch)
+    refs = [oracle.PreCorr(f.order, np.array(f.a), np.array(f.g), limit) for _ in range(nch)]
+    got = gpu.process_block(torch.from_numpy(ahead).cuda(), first=0)[0].cpu().numpy()
+    np.testing.assert_array_equal(got, refs[0].process(ahead))
+    for lo, hi in ((0, 1500), (1500, n)):
+        got = gpu.process_block(torch.from_numpy(x[:, lo:hi].copy()).cuda()).cpu().numpy()
+        for c in range(nch):
+            np.testing.assert_array_equal(got[c], refs[c].process(x[c, lo:hi]), err_msg=f"{c} {lo}")
