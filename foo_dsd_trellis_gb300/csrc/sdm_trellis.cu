@@ -206,9 +206,17 @@ static int child_ops(int N, int H, bool im) {
 //   K = 4:  608 jobs 1,879 / 2,607 at 32 / 16, 1,216 jobs 3,154 / 2,675 / 2,570
 //           at 32 / 16 / 8, 4,000 jobs 3,189 at 8
 //   K = 8:  1 job 2,396 / 2,507 at 32 / 16, 608 jobs 2,504 / 2,525, 1,216 jobs 4,414 / 2,567
+// At K <= 2 the per-thread kernel (32 jobs a warp) is the alternative, from 5
+// warps of eight jobs a scheduler on, at K = 1 from 3 (the second wave); us a
+// step, child / per-thread kernel:
+//   K = 2: order 4 12,000 jobs 1.56 / 3.25, 24,000 3.02 / 3.48, 32,000 4.45 / 4.00;
+//          order 6 12,000 2.05 / 3.91, 24,000 3.95 / 4.25; order 8 24,000 4.88 / 5.08
+//   K = 1: order 8 12,000 2.53 / 3.79, 18,000 4.86 / 4.05, 24,000 4.88 / 4.86
+// At K = 3, 4 there is none: the warp kernel, eight jobs a warp, took 5.8 us at
+// 8,000 jobs of order 6 and 12.2 at 20,000, this one 3.6 and 7.2.
 // The warp kernel's step (one candidate a lane, its selection in sequence with
 // its arithmetic) takes 5,500 cycles alone and 8,925 at order 8 with 2.47 warps
-// a scheduler (the child kernel 5,700); the per-thread kernel (K <= 2) 9,600.
+// a scheduler (the child kernel 5,700).
 static int child_lanes(const SdmParams& P, int njobs) {
   const int K = P.cands, N = P.order;
   if (K > 16) return 0;
@@ -226,10 +234,9 @@ static int child_lanes(const SdmParams& P, int njobs) {
     const double c = std::max(66.0 * ops + alone, 76.0 * ops * w + 650.0);
     if (c < cost) { cost = c; best = lanes; }
   }
+  if (K <= 2) return warps(8) > (K == 1 ? 3.0 : 5.0) && sdm_scalar_eligible(P, 0) ? 0 : best;
   double other = 1e300;
-  if (K <= 2) {
-    other = std::max(9600.0, 76.0 * K * (5.0 * N + 6.0) * warps(32));
-  } else if (K > 4 && P.lat <= 32 * kRegRingWords) {
+  if (K > 4 && P.lat <= 32 * kRegRingWords) {
     const int lanes = min_lanes(K);
     const double slots = pipes / 4.0 * 10.0;
     const int groups = (int)std::min(32.0 / lanes, std::max(1.0, std::ceil(njobs / slots)));

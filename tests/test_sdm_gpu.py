@@ -625,3 +625,43 @@ def test_runaway_modulator_warp_kernel(oracle, K, depth, lanes, name, rate, amp,
     assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
         (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"])
     np.testing.assert_array_equal(q["best_state"], ref.best_state())
+
+
+@pytest.mark.parametrize("K,depth,order", [(2, 4, 6), (1, 6, 4), (2, 6, 8)])
+def test_per_thread_kernel_shares_the_context_format(oracle, K, depth, order):
+    """Contexts carried through the per-thread kernel (more jobs than five warps
+    of eight a scheduler), the child kernel (few of them), the warp kernel at 2
+    and 32 lanes, and the first two again; each call continues from the last."""
+    from foo_dsd_trellis_gb300 import _lib
+    f = _ntf({4: "clans-4", 6: "clans-6", 8: "clans-8"}[order], 5644800)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    many = 5 * 8 * 4 * sms + 33
+    g = _gpu_sdm(f, depth, K, 32, nctx=many)
+    refs = [_ora(oracle, f, depth, K, 32) for _ in range(2)]
+    x = np.stack([multitone(2200, seed=90 + c) * 0.7 for c in range(2)])
+    at = [0, many - 1]
+    pos = 0
+    for stage, ln in (("all", 333), ("few", 300), ("lanes2", 310), ("lanes32", 290), ("all", 400), ("few", 350)):
+        blk = x[:, pos:pos + ln]
+        pos += ln
+        g.set_option(_lib.OPT_SDM_LANES, {"lanes2": 2, "lanes32": 32}.get(stage, 0))
+        if stage == "all":
+            xa = torch.zeros((many, ln), dtype=torch.float64, device="cuda")
+            for c in range(2):
+                xa[at[c]] = torch.from_numpy(blk[c].copy()).cuda()
+            out = g.process_block(xa)
+            got = [out[i] for i in at]
+        else:
+            got = [g.process_block(torch.from_numpy(blk[c].copy()).cuda(), first=at[c])[0] for c in range(2)]
+        want = {"all": "sdm_scalar_kernel", "few": "sdm_child_kernel"}.get(stage, "sdm_jobs_kernel")
+        assert g.last_sdm_kernel().startswith(want), stage
+        for c in range(2):
+            np.testing.assert_array_equal(got[c].cpu().numpy(), oracle.sdm_bits(refs[c], blk[c]), err_msg=stage)
+    g.set_option(_lib.OPT_SDM_LANES, 0)
+    for c in range(2):
+        q, info = g.query(at[c]), refs[c].info()
+        assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
+            (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"])
+        np.testing.assert_array_equal(q["best_state"], refs[c].best_state())
+        got = g.drain(64, at[c], 1)[0].cpu().numpy()
+        np.testing.assert_array_equal(got, (refs[c].drain(64) > 0).astype(np.uint8))
