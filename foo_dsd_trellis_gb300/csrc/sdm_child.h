@@ -429,23 +429,8 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
   load_x(kBlock);
   double d[C], v = 0.0;
   const bool stored = !(job.flags & kJobNoStore);
-  if (n_in == 0 && has && stored && r < n) {
-    // no samples: the (copied, seeded) state as it is
-    if (b == 0) {
-#pragma unroll
-      for (int j = 0; j < C; j++)
-        if (q * C + j < N) dst->s[r][q * C + j] = s[j];
-      if (q == 0) {
-        dst->cost[r] = cost;
-        dst->path[r] = path;
-        dst->next[r] = (uint8_t)nxt;
-        dst->slot[r] = (uint8_t)r;
-        for (int w = 0; w < W; w++) dst->ring[r][w] = ring[w * KC + r];
-      }
-    }
-  }
   __syncwarp();
-  if (n_max > 0) advance<N, H, C, false>(P, s, s_x[js][0], d, v, gl, al, s[0], q, lane0, zg, [](int) {});
+  advance<N, H, C, false>(P, s, s_x[js][0], d, v, gl, al, s[0], q, lane0, zg, [](int) {});
 
   // steps from step t to the next at which a job leaves its ring's word or ends
   auto next_event = [&](long long t) {
@@ -788,15 +773,6 @@ sdm_child_kernel(const __grid_constant__ SdmParams P, const SdmJob* __restrict__
       dst->skey[bk][j] = src->skey[bk][j];
       dst->slink[bk][j] = src->slink[bk][j];
     }
-  }
-  if (n_in == 0 && has && stored && jl == 0) {
-    dst->n = n;
-    dst->bank = bank0;
-    dst->pos = pos;
-    dst->conv_fail = c_conv;
-    dst->cands_collapse = c_coll;
-    dst->next_filter_drops = c_drop;
-    dst->total_children = c_tot;
   }
   err = __reduce_max_sync(kFull, err);
   if (err && wl == 0) atomicMax(status, err);

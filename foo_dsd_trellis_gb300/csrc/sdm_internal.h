@@ -89,7 +89,9 @@ struct alignas(16) SdmCtx {
 // through context `ctx`, dropping the decisions of the first `skip_out` steps
 // and writing the rest as 0/1 bytes to `out`.  Optionally the context is
 // first copied from `copy_from` (sdm_context_copy_state) and its live
-// candidates seeded with `seed_state` and zero cost (DAS temp seeding).
+// candidates seeded with `seed_state` and zero cost (DAS temp seeding).  A job
+// has at least one sample: the kernels store a context at its last one, and the
+// host does what an empty one asks for without a job.
 struct SdmJob {
   const double* in;       // nullptr: zeros (drain)
   uint8_t* out;

@@ -665,3 +665,35 @@ def test_per_thread_kernel_shares_the_context_format(oracle, K, depth, order):
         np.testing.assert_array_equal(q["best_state"], refs[c].best_state())
         got = g.drain(64, at[c], 1)[0].cpu().numpy()
         np.testing.assert_array_equal(got, (refs[c].drain(64) > 0).astype(np.uint8))
+
+
+@pytest.mark.parametrize("K,depth,lat,njobs,order", [(2, 4, 70, 900, 6), (2, 6, 9, 2500, 7), (4, 8, 33, 1400, 5),
+                                                     (8, 16, 100, 1300, 8), (16, 32, 65, 6, 6), (16, 9, 300, 40, 7)])
+def test_contexts_of_uneven_jobs_continue(oracle, K, depth, lat, njobs, order):
+    """Jobs of uneven lengths beside one another in a warp: the context that each
+    leaves (its ring and place in it among the rest) goes on as the oracle's."""
+    from foo_dsd_trellis_gb300.sdm import SegmentSpec
+    f = _ntf({5: "clans-5", 6: "clans-6", 7: "clans-7", 8: "clans-8"}[order], 5644800)
+    lens = [1, 31, 32, 33, 64, 97, 130, 400]
+    x = multitone(1500, seed=K + njobs) * 0.8
+    g = _gpu_sdm(f, depth, K, lat, nctx=njobs + 1)
+    base = _ora(oracle, f, depth, K, lat)
+    oracle.sdm_bits(base, x[:333])
+    g.process_block(torch.from_numpy(x[:333].copy()).cuda(), first=njobs)
+    xs = torch.from_numpy(x).cuda()
+    at = lambda i: (lens[(i * 5 + i // 8) % len(lens)], 333 + i % 200)
+    g.segments([SegmentSpec(xs[at(i)[1]:at(i)[1] + at(i)[0]], channel=i, seed_from=njobs) for i in range(njobs)])
+    assert g.last_sdm_kernel().startswith("sdm_child_kernel")
+    more = x[1000:1300]
+    outs = g.process_block(torch.from_numpy(np.repeat(more[None], njobs, 0)).cuda())
+    for i in list(range(min(njobs, 20))) + list(range(20, njobs, 97)):
+        n, lo = at(i)
+        ctx = _ora(oracle, f, depth, K, lat)
+        ctx.copy_from(base)
+        oracle.segment_bits(ctx, x[lo:lo + n], 0)
+        np.testing.assert_array_equal(outs[i].cpu().numpy(), oracle.sdm_bits(ctx, more), err_msg=str(i))
+        q, info = g.query(i), ctx.info()
+        assert (q["num_cands"], q["total_children"], q["next_filter_drops"], q["conv_fail"]) == \
+            (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"]), i
+        np.testing.assert_array_equal(g.drain(lat + 5, i, 1)[0].cpu().numpy(),
+                                      (ctx.drain(lat + 5) > 0).astype(np.uint8))
