@@ -254,7 +254,9 @@ int launch_sdm_jobs(const SdmParams& P0, const SdmJob* d_jobs, int njobs, int* d
                     SdmCtx* d_ctxs, int* d_status, int max_blocks, cudaStream_t stream) {
   if (njobs <= 0) return 0;
   const SdmParams P = with_int(P0);
-  if (P.lanes == 0 && max_blocks == 0) {
+  // (a path-hash walk that gives up early, DSDGPU_FAIL_CHAIN_WALK, is the warp
+  // kernel's above K = 4: the child kernel walks no chain)
+  if (P.lanes == 0 && max_blocks == 0 && !(P.hop_limit > 0 && P.cands > 4)) {
     const int cl = child_lanes(P, njobs);
     if (cl > 0) {
       const int KC = P.cands <= 2 ? 2 : P.cands <= 4 ? 4 : P.cands <= 8 ? 8 : 16;

@@ -84,3 +84,28 @@ def test_failure_test_option_rejects_unknown_bits():
     g = TrellisSdm(f.order, f.a, f.g, 8, 4, 16, num_contexts=1)
     assert g.L.dsdgpu_set_option(g.h, _lib.OPT_FAILURE_TEST, 4) == _lib.ERR_ARG
     g.close()
+
+
+@pytest.mark.parametrize("K", [8, 16])
+def test_chain_walk_bound_below_k17(oracle, K):
+    """The same bound at K = 5 .. 16, whose launches otherwise take a kernel that
+    walks no chain."""
+    from foo_dsd_trellis_gb300 import _lib
+    from foo_dsd_trellis_gb300.sdm import TrellisSdm
+    f = _ntf("clans-7", 6144000)
+    depth, lat = 64, 64
+    x = np.stack([multitone(20000, 41) * 2.0, multitone(20000, 42) * 2.0])
+    g = TrellisSdm(f.order, f.a, f.g, depth, K, lat, num_contexts=2)
+    g.set_select(_lib.SELECT_EXACT)
+    g.set_option(_lib.OPT_FAILURE_TEST, _lib.FAIL_CHAIN_WALK)
+    with pytest.raises(_lib.DsdGpuError) as err:
+        g.process_block(torch.from_numpy(x).cuda())
+    assert err.value.code == _lib.ERR_DEVICE
+    g.set_option(_lib.OPT_FAILURE_TEST, 0)
+    _lib.check(g.h, g.L.dsdgpu_sdm_reset(g.h, -1))
+    got = [t.cpu().numpy() for t in g.process_block(torch.from_numpy(x).cuda())]
+    assert g.last_sdm_kernel().startswith("sdm_child_kernel")
+    g.close()
+    for c in range(2):
+        ref = oracle.sdm(f.order, np.array(f.a), np.array(f.g), depth, K, lat)
+        assert np.array_equal(got[c], oracle.sdm_bits(ref, x[c]))
