@@ -324,14 +324,14 @@ int measure_curve(dsdgpu_context* c, const SdmParams& P, TuneCurve* out) {
     SdmParams Q = P;
     Q.mode = c->sdm_mode;
     Q.lanes = lanes_per_job(P);   // the width the plan's capped launches use
-    // warm-up
-    if (launch_sdm_jobs(Q, d_j, sms * jpc, d_cnt, d_c, c->d_status, 0, c->stream) != 0)
+    // warm-up (capped launches, as the plan's are: the cap picks the build)
+    if (launch_sdm_jobs(Q, d_j, sms * jpc, d_cnt, d_c, c->d_status, sms, c->stream) != 0)
       rc = c->cuda_fail(cudaGetLastError(), "tuner launch");
     for (int lv : kTuneWarpLevels) {
       if (rc) break;
       const int w = lv * sms * jpc;            // resident jobs (lv warps per SM)
       cudaEventRecord(e0, c->stream);
-      if (launch_sdm_jobs(Q, d_j, w, d_cnt, d_c, c->d_status, 0, c->stream) != 0) {
+      if (launch_sdm_jobs(Q, d_j, w, d_cnt, d_c, c->d_status, lv * sms, c->stream) != 0) {
         rc = c->cuda_fail(cudaGetLastError(), "tuner launch");
         break;
       }
