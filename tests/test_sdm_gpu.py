@@ -697,3 +697,40 @@ def test_contexts_of_uneven_jobs_continue(oracle, K, depth, lat, njobs, order):
             (info["num_cands"], info["total_children"], info["next_filter_drops"], info["conv_fail"]), i
         np.testing.assert_array_equal(g.drain(lat + 5, i, 1)[0].cpu().numpy(),
                                       (ctx.drain(lat + 5) > 0).astype(np.uint8))
+
+
+@pytest.mark.parametrize("levels", [3, 16, 32, 97])
+@pytest.mark.parametrize("a0", [-0.9, 1e-120, -1e-120, 3e110])
+def test_estimate_state_unusual_a0(oracle, levels, a0):
+    """The estimator's thresholds with a negative a_0 (the order of the levels
+    turned round), and a_0 too small or large for thresholds, where every block
+    takes the reference's divisions: equal to the oracle with and without the
+    limiter, over counts around the blocks of 32."""
+    import ctypes as C
+    from foo_dsd_trellis_gb300 import _lib
+    L = _lib.load()
+    h = C.c_void_p()
+    assert L.dsdgpu_create(0, C.byref(h)) == 0
+    f = _ntf("clans-6", 5644800)
+    a = [a0] + list(f.a[1:])
+    rng = np.random.default_rng(levels)
+    for lim in (0.0, 1.5):
+        p = _lib.SdmParams()
+        p.order = f.order
+        for i in range(f.order):
+            p.a[i], p.g[i] = a[i], f.g[i]
+        p.state_limit = lim
+        counts = [1, 31, 32, 33, 500]
+        xs = [0.3 * rng.standard_normal(n) for n in counts]
+        d_x = [torch.from_numpy(x).cuda() for x in xs]
+        items = (_lib.EstimateItem * len(counts))()
+        inits = [rng.standard_normal(f.order) * 0.1 for _ in counts]
+        for j, n in enumerate(counts):
+            items[j].d_in, items[j].count = d_x[j].data_ptr(), n
+            for k in range(f.order):
+                items[j].init_state[k] = inits[j][k]
+        _lib.check(h, L.dsdgpu_sdm_estimate_state(h, C.byref(p), levels, items, len(counts)))
+        for j, n in enumerate(counts):
+            want = oracle.estimate_state(f.order, np.array(a), np.array(f.g), inits[j], xs[j], lim, levels)
+            np.testing.assert_array_equal(np.array(items[j].out_state[: f.order]), want, err_msg=f"{lim} {n}")
+    L.dsdgpu_destroy(h)
