@@ -34,8 +34,9 @@ static int resident_warps() {
 
 // Lanes and jobs per warp of a launch of njobs jobs with no block cap: the
 // tightest width, and the fewest jobs a warp that still let every job start at
-// once (warp slots: 16 one-warp CTAs per SM at 32 lanes, 10 below, whose launch
-// bound leaves up to 204 registers).  The selection's sort is as deep as the
+// once (warp slots: 16 one-warp CTAs per SM at 32 lanes, 12 below, whose builds
+// take up to 168 registers; counted as 10, 1,700 jobs at K = 16 went two a warp,
+// order 7 3.47 us a step against 2.63).  The selection's sort is as deep as the
 // width asks (21 exchanges at 32 lanes, 15 at 16, 10 at 8), and an FP64
 // instruction costs the same with 8 lanes active as with 32, so idle lanes
 // beside a job cost nothing while a second job on them costs its FP64 time.
@@ -44,7 +45,7 @@ static int launch_lanes(const SdmParams& P, int njobs, int max_blocks, int* grou
   *groups = 32 / lanes;
   if (P.lanes > 0 || max_blocks > 0 || P.lat > 32 * kRegRingWords) return lanes;
   lanes = min_lanes(P.cands);
-  const long long slots = (long long)(resident_warps() / 16) * (lanes == 32 ? 16 : 10);
+  const long long slots = (long long)(resident_warps() / 16) * (lanes == 32 ? 16 : 12);
   *groups = (int)std::min<long long>(32 / lanes, std::max<long long>(1, (njobs + slots - 1) / slots));
   return lanes;
 }
@@ -238,7 +239,7 @@ static int child_lanes(const SdmParams& P, int njobs) {
   double other = 1e300;
   if (K > 4 && P.lat <= 32 * kRegRingWords) {
     const int lanes = min_lanes(K);
-    const double slots = pipes / 4.0 * 10.0;
+    const double slots = pipes / 4.0 * 12.0;
     const int groups = (int)std::min(32.0 / lanes, std::max(1.0, std::ceil(njobs / slots)));
     other = std::max(5500.0, 89.0 * 5.0 * N * warps(groups));
   }

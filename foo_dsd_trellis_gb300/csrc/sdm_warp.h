@@ -39,12 +39,11 @@
 namespace dsdgpu {
 
 // One warp per CTA (one job, or 32 / LPJ jobs side by side for K <= 16): a
-// few thousand long-running jobs spread evenly over the SMs.  At 32 lanes the
-// launch bound (32 threads, 13 CTAs per SM) holds the kernel at 128 registers
-// (a 152-register build measured 50 % slower on the DSD128 DAS workload, with
-// fewer warps per FP64 pipe); narrower widths take 10 CTAs per SM, which left
-// the 16-lane order-8 kernel at 168 registers with 60 bytes of spills instead
-// of 344 and ran the DSD512 workload 6.7 % faster (442.1 -> 471.5).
+// few thousand long-running jobs spread evenly over the SMs.  At 32 lanes a
+// launch bound of 13 CTAs per SM holds the kernel at 128 registers (up to 112
+// bytes of spills), one of 12 at 168 without spills, for launches that fit it;
+// at narrower widths the compiler takes at most 168 (up to 36 bytes of spills at
+// orders 7 to 10), of which 12 CTAs fit.
 constexpr int kRegRingWords = 8;      // rings held in registers: lat <= 256
 constexpr unsigned kFull = 0xffffffffu;
 
