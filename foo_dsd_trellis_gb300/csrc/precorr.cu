@@ -336,8 +336,14 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, bool plain, PcSta
   float xa[kPcAhead];
 #pragma unroll
   for (int j = 0; j < kPcAhead; j++) xa[j] = j < count ? x[j] : 0.0f;
+  // Channels that run side by side take the same kind of step: one whose chunk
+  // does not stand takes the others with it (both kinds in one warp cost the
+  // sum).  One of 2 / 32 channels at the limiter, order 8, ns a sample: 136 / 170
+  // each for itself, 60 / 77 together; every channel in whole steps 60 / 76, in
+  // short ones 45 / 63.
+  plain = __all_sync(__activemask(), plain);
   long long base = 0;
-  int hold = 0;   // chunks to go in whole steps after one that did not stand
+  long long until = 0;   // whole steps up to here after a chunk that did not stand
   // whole chunks: straight-line code over kPcAhead samples, the next chunk's
   // inputs in flight meanwhile (converted when used)
   for (; base + kPcAhead <= count; base += kPcAhead) {
@@ -354,13 +360,7 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, bool plain, PcSta
     }
     unsigned w[kPcAhead / 4] = {0u, 0u, 0u, 0u};
     bool stands = false;
-    // channels that run side by side take the same kind of step: one whose chunk
-    // does not stand takes the others with it, which costs them the whole step
-    // (both kinds in one warp cost the sum).  One of 2 / 32 channels at the
-    // limiter, order 8, ns a sample: 136 / 140 apart, 60 / 77 together; every
-    // channel in whole steps 60 / 77, in short ones 45 / 59.
-    const unsigned side = __activemask();
-    if (__all_sync(side, plain && hold == 0)) {
+    if (plain && base >= until) {
       float keep[N];
 #pragma unroll
       for (int k = 0; k < N; k++) keep[k] = W.s[k];
@@ -371,7 +371,7 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, bool plain, PcSta
         pc_plain_step<N, LIM>(W, xa[j], y, peak);
         neg = __funnelshift_l(__float_as_uint(y), neg, 1);
       }
-      stands = __all_sync(side, pc_stands<N, LIM>(W, peak));
+      stands = __all_sync(__activemask(), pc_stands<N, LIM>(W, peak));
       if (stands) {
         W.hist = ~neg & 0xffu;
         W.pbit = ~neg & 1u;
@@ -381,10 +381,8 @@ __device__ void pc_run(const PcCoef& Cg, const uint8_t* codes, bool plain, PcSta
       } else {
 #pragma unroll
         for (int k = 0; k < N; k++) W.s[k] = keep[k];
-        hold = kPcHold;
+        until = base + (kPcHold + 1) * kPcAhead;
       }
-    } else if (hold > 0) {
-      hold--;
     }
     if (!stands) {
 #pragma unroll
