@@ -9,7 +9,8 @@
 // the inputs cut into blocks X[n] of B = max(D, 16), an output is
 //   y[n] = sum_j sum_r h[B j - r] X[n - j][r]
 // a matrix product with the taps on one side and decisions on the other.  The
-// taps are taken to 2^-55 of their scale or finer and cut into seven 8-bit
+// taps are rounded to fixed point (to 2^-55 of the largest up to D = 128, 2^-54
+// at 256, 2^-53 at 512, where the last bit is 2^-61) and cut into seven 8-bit
 // digits, which bf16 holds exactly; every partial sum is a whole number below
 // 2^24, so the tensor cores' FP32 accumulators are exact, and the digits' sums
 // are joined as 64-bit integers.  Only the taps' own rounding is left (an FP64
@@ -635,7 +636,8 @@ int form_taps(dsdgpu_context_t* c, dsdgpu_decim_state* s) {
   cudaMemcpyAsync(&peak, d_peak, sizeof peak, cudaMemcpyDeviceToHost, c->stream);
   const cudaError_t e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return c->cuda_fail(e, "decimation taps");
-  // the digits' sum stays below 2^63 (sum |h| < 1.9), a tap below 2^54
+  // a tap stays below 2^54 (seven digits), and with at most 61 the joined sum
+  // below 1.9 x 2^61, a bit within 64 (sum |h| < 1.9 at every ratio)
   s->mma.shift = 61;
   while (std::ldexp(peak, s->mma.shift) > std::ldexp(1.0, 54)) s->mma.shift--;
   decim_frag_kernel<<<nb(words, 256), 256, 0, c->stream>>>(s->mma, 1 << s->stages, h, len,

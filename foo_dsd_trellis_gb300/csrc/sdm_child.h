@@ -29,7 +29,7 @@
 //   v = ((x + p_0) + p_1) + ...;  children: s_0 = d_0 +- 1, e = v +- a_0
 // (adding -m is subtracting m, adding -0.0 leaves any value as it is).  The
 // products with the filter's structurally zero g are left out while every v
-// is finite (see sdm_trellis.cu).
+// is finite (see sdm_warp.h).
 //
 // What bounds a step now is its FP64 instructions (child_ops in
 // sdm_trellis.cu, 64 cycles each) and about 500 cycles of the selection that

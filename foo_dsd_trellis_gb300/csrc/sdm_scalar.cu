@@ -3,8 +3,8 @@
 //
 // On this part an FP64 warp instruction occupies the FP64 unit about as long
 // with 2 active lanes as with 32, so a warp-cooperative job at K = 2 (the
-// kernel in sdm_trellis.cu) spends a full warp instruction on every
-// operation of 2 candidates, and its sort, ballots and shuffles sit on the
+// kernels in sdm_warp.h and sdm_child.h) spends a warp instruction on every
+// operation of a few candidates, and its sort, ballots and shuffles sit on the
 // per-sample critical path.  Here every lane carries its own job: each FP64
 // instruction advances 32 jobs, and the selection of at most 4 children is a
 // few predicated integer operations in registers.

@@ -10,12 +10,13 @@
 //                  no contraction: __dadd_rn/__dmul_rn) and forms both
 //                  children: slots 2i (bit 0, state[0] + 1) and 2i + 1
 //                  (bit 1, state[0] - 1)          (reference src/trellis.c:37-191)
-//   2. selection   warp argmin over the 2n children by int64 cost bits,
-//                  majority vote on the traceback bit with the 1.1x override,
-//                  then the reference's ordered insertion with path-hash
-//                  dedup, emulated warp-cooperatively: the sorted act list is
-//                  held one entry per lane and every insertion is a ballot +
-//                  shuffle; the hash chains are walked in shared memory
+//   2. selection   the 2n children sorted by int64 cost bits and index, as
+//                  one 32-bit word each where those tell, the whole pairs
+//                  where they do not; majority vote on the traceback bit with
+//                  the 1.1x override; without equal paths the sorted
+//                  positions of the eligible children are their ranks, else
+//                  the reference's ordered insertion with path-hash dedup,
+//                  the hash chains walked in shared memory
 //                                                  (src/trellis.c:582-731)
 //   3. commit      survivors pull their parent's state, path, traceback bit
 //                  and ring with shuffles, normalise cost by the new minimum
