@@ -59,8 +59,8 @@ WL = dict(workload="dsd128_das_stereo_10s_multitone_pink", fs_in=48000, fs_out=6
 FP64_OPS_PER_CAND_SAMPLE = 5 * WL["ntf_order"] + 6   # (2N+1) mul + (3N+5) add
 MEASURED_BF16_TFLOPS = 1926.4                         # MEASURED_PEAKS.json bf16_tflops
 FP64_ISSUED_PER_CAND_SAMPLE = 27                      # of them on the FP64 unit at N = 7
-SDM_DRAM_BYTES_PER_SAMPLE = 9.04                      # measured, see the traffic note below
-SDM_PARTS_DRAM_BYTES_PER_SAMPLE = 9.15                # the balanced launch's (parts kernel), measured
+SDM_DRAM_BYTES_PER_SAMPLE = 9.00                      # measured, see the traffic note below
+SDM_PARTS_DRAM_BYTES_PER_SAMPLE = 9.12                # the balanced launch's (parts kernel), measured
 
 
 # The rows beside the headline, measured by the default run as well: the
@@ -1081,7 +1081,7 @@ def run_conv(args):
                              "peak": fp64_peak / 1000.0, "unit": "TFLOP/s",
                              "frac": flops / sdm_s / 1e12 / (fp64_peak / 1000.0),
                              "traffic": SDM_DRAM_BYTES_PER_SAMPLE * sdm_samples,
-                             "traffic_source": "9.04 B per SDM input sample (ncu, sdm_jobs_kernel "
+                             "traffic_source": "9.00 B per SDM input sample (ncu, sdm_jobs_kernel "
                                                "at K = 32), scaled by SDM input samples",
                              "kernel": enc.last_sdm_kernel()},
                 "cpu_baseline": None, "clocks": clk, "gpu_launches": int(launches),

@@ -22,7 +22,7 @@
 // fragment; a warp uses each fragment for two digits, since making it (three
 // half-rate integer instructions) takes as long as a product (mma.sync
 // m16n8k16: 8.35 cycles a scheduler, measured).  What bounds it: the tensor
-// pipe (active half of the time, ncu; 448 multiply-adds an input decision),
+// pipe (active 60 % of the time, ncu; 448 multiply-adds an input decision),
 // then the taps' loads from L2.  10 s of stereo DSD128 to 44.1 kHz, the whole
 // call: 4,560 us stage by stage, 343 us here (7 warps of one digit over all
 // columns 573, prmt by an intrinsic that masks its selector 577, one digit a
